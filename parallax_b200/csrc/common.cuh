@@ -48,15 +48,21 @@ struct ViewDesc {
   int32_t gauss_count;
 };
 
-// Per-step screen-space gradient accumulators of one (view, gaussian) slot
-// (the per-splat vectors of SplatRaster.cpp:337-342), 12 floats, 16-byte aligned.
+// Per-step screen-space gradient accumulators of one (view, gaussian) slot, 12
+// floats, 16-byte aligned. With p the power of a pixel's exponent and
+// z = dL/dp there (0 where the alpha cap flattens it), the per-splat vectors of
+// SplatRaster.cpp:337-342 are linear in six moments of z over the pixels, with
+// the splat's conic (a, b, c) and opacity o as constants, so the adjoint sums
+// the moments and the parameter chain applies the constants once per slot:
+//   dL/dmean  = (a Sx + b Sy, b Sx + c Sy)
+//   dL/dconic = (-Sxx / 2, -Sxy, -Syy / 2)
+//   dL/do     = S0 / o
 struct alignas(16) ScreenGrad {
-  float dmean[2];
-  float dconic[3];
-  float dopacity;
+  float s0, sx, sxx;  // sums of z, z dx, z dx^2 (dx, dy: pixel centre - mean)
+  float sy, sxy, syy;
   float dcolor[3];
-  float dmean_abs;
-  float touched;  // 1 when any pixel reached the uncapped-alpha branch
+  float dmean_abs;  // sum of |dL/dmean| per pixel, the densify statistic
+  float touched;  // nonzero when any pixel reached the uncapped-alpha branch
   float pad;
 };
 static_assert(sizeof(ScreenGrad) == 48, "ScreenGrad layout");

@@ -143,9 +143,9 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
   covariance(Rg, sc, Sigma, Mg);
   const pxs_camera& cam = vd.cam;
   const uint32_t clamped = __float_as_uint(col.w);
-  // opacity: alpha = sigmoid(logit) * G
+  // opacity: alpha = sigmoid(logit) * G, dL/do = s0 / o
   const float opacity = co.w;
-  out[PXS_C_OPACITY * kParamThreads] = sg.dopacity * opacity * (1.f - opacity);
+  out[PXS_C_OPACITY * kParamThreads] = sg.s0 * (1.f - opacity);
   // colour: through the SH clamp into the coefficients and the direction
   float dcol[3];
 #pragma unroll
@@ -192,11 +192,11 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
            cam.t[i];
   const float z = p[2];
   const float fx = cam.fx, fy = cam.fy;
-  const float dmx = sg.dmean[0], dmy = sg.dmean[1];
+  const float dmx = co.x * sg.sx + co.y * sg.sy, dmy = co.y * sg.sx + co.z * sg.sy;
   float dp[3] = {fx / z * dmx, fy / z * dmy, -(fx * p[0] * dmx + fy * p[1] * dmy) / (z * z)};
   // conic -> 2D covariance: -(A D A), D the symmetric gradient
   const float A[4] = {co.x, co.y, co.y, co.z};
-  const float Dm[4] = {sg.dconic[0], 0.5f * sg.dconic[1], 0.5f * sg.dconic[1], sg.dconic[2]};
+  const float Dm[4] = {-0.5f * sg.sxx, -0.5f * sg.sxy, -0.5f * sg.sxy, -0.5f * sg.syy};
   float AD[4], dcov2[4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)

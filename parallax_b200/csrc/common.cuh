@@ -49,17 +49,20 @@ struct ViewDesc {
 };
 
 // Per-step screen-space gradient accumulators of one (view, gaussian) slot, 12
-// floats, 16-byte aligned. With p the power of a pixel's exponent and
-// z = dL/dp there (0 where the alpha cap flattens it), the per-splat vectors of
-// SplatRaster.cpp:337-342 are linear in six moments of z over the pixels, with
-// the splat's conic (a, b, c) and opacity o as constants, so the adjoint sums
-// the moments and the parameter chain applies the constants once per slot:
-//   dL/dmean  = (a Sx + b Sy, b Sx + c Sy)
-//   dL/dconic = (-Sxx / 2, -Sxy, -Syy / 2)
-//   dL/do     = S0 / o
+// floats, 16-byte aligned. With z = dL/dp of a pixel's power p = -1/2 d^T A d
+// (0 where the alpha cap flattens it), d its centre less the mean, A the
+// splat's conic, o its opacity and (u, w) = A d, the per-splat gradients of
+// SplatRaster.cpp:337-342 and 455-470 are
+//   dL/dmean  = sum of z (u, w)
+//   dL/dcov2d = -A (dL/dA) A = 1/2 sum of z (u, w)^T (u, w)
+//   dL/do     = sum of z / o
+// Sums of z d^T d, dL/dA, would be multiplied by A afterwards; in an elongated
+// splat that cancels all but (minor / major axis)^2 of them and brings up the
+// rounding of the FP32 sums, while A d cancels pixel by pixel, before the sum.
 struct alignas(16) ScreenGrad {
-  float s0, sx, sxx;  // sums of z, z dx, z dx^2 (dx, dy: pixel centre - mean)
-  float sy, sxy, syy;
+  float s0;         // sum of z
+  float dcov[3];    // sums of z u^2, z u w, z w^2
+  float dmean[2];
   float dcolor[3];
   float dmean_abs;  // sum of |dL/dmean| per pixel, the densify statistic
   float touched;  // nonzero when any pixel reached the uncapped-alpha branch

@@ -192,21 +192,11 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
            cam.t[i];
   const float z = p[2];
   const float fx = cam.fx, fy = cam.fy;
-  const float dmx = co.x * sg.sx + co.y * sg.sy, dmy = co.y * sg.sx + co.z * sg.sy;
+  const float dmx = sg.dmean[0], dmy = sg.dmean[1];
   float dp[3] = {fx / z * dmx, fy / z * dmy, -(fx * p[0] * dmx + fy * p[1] * dmy) / (z * z)};
-  // conic -> 2D covariance: -(A D A), D the symmetric gradient
-  const float A[4] = {co.x, co.y, co.y, co.z};
-  const float Dm[4] = {-0.5f * sg.sxx, -0.5f * sg.sxy, -0.5f * sg.sxy, -0.5f * sg.syy};
-  float AD[4], dcov2[4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) AD[i * 2 + j] = A[i * 2 + 0] * Dm[0 * 2 + j] + A[i * 2 + 1] * Dm[1 * 2 + j];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      dcov2[i * 2 + j] = -(AD[i * 2 + 0] * A[0 * 2 + j] + AD[i * 2 + 1] * A[1 * 2 + j]);
+  // the 2D covariance's gradient, symmetric (see ScreenGrad)
+  const float dcov2[4] = {0.5f * sg.dcov[0], 0.5f * sg.dcov[1], 0.5f * sg.dcov[1],
+                          0.5f * sg.dcov[2]};
   // 2D covariance -> 3D covariance and the projection Jacobian
   float J[6], T[6];
   jacobian_times_w(p, cam, J, T);

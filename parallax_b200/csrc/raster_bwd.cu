@@ -4,12 +4,12 @@
 // walks its tile's list back to front from its last contributor (recorded by
 // the forward kernel), dividing the transmittance back out rather than storing
 // it per pair, and the per-splat screen-space gradients are summed over the
-// tile's pixels as moments of dL/dpower (ScreenGrad), the colour gradient and
-// the densify statistic:
-//   * per warp with an 11-shuffle transpose reduction (warp_reduce_moments);
+// tile's pixels (ScreenGrad):
+//   * per warp and two entries at a time with a 21-shuffle transpose reduction
+//     (warp_reduce);
 //   * once per (warp, splat) into global memory: each of eleven lanes holds one
 //     complete sum and adds it to its float of the slot's accumulators, one
-//     reduction instruction over 44 consecutive bytes.
+//     reduction instruction for both entries.
 // The branch decisions (power > 0, the alpha floor, the 0.99 cap) are taken
 // with the forward kernel's exact rounding (raster_common.cuh); the gradient
 // arithmetic itself may use fused multiply-adds.
@@ -28,67 +28,66 @@ __device__ __forceinline__ void red_add(float* address, float x) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(address), "f"(x) : "memory");
 }
 
-// One entry's sums over a lane's pixels, all in one column: z, z dy, z dy^2,
-// the colour gradient, |dmean|.
+// One entry's sums over a lane's pixels (ScreenGrad): z; z u^2, z u w, z w^2;
+// z u, z w; the colour gradient; |dmean|.
 struct LaneSums {
-  float a0, a1, a2, c0, c1, c2, ab;
+  float z, uu, uw, ww, u, w, c0, c1, c2, ab;
 };
 
-// Where a lane's result of warp_reduce_moments belongs: the float of the slot's
-// ScreenGrad, or -1.
-__device__ __forceinline__ int moment_index(int lane) {
-  const int group = lane >> 3;
-  const int out = (lane & 4) == 0 ? ((lane & 3) == 0 ? 0 : -1)
-                                  : ((lane & 1) == 0 ? 1 + ((lane >> 1) & 1) : -1);
-  if (out < 0 || (group == 2 && out == 2)) return -1;
-  // group 0: s0, sx, sxx; 1: sy, sxy, syy; 2: dmean_abs, touched; 3: dcolor
-  return group < 2 ? 3 * group + out : group == 2 ? 9 + out : 6 + out;
+// Where a lane's result of warp_reduce belongs: the float of the slot's
+// ScreenGrad, or -1. Lanes 0-15 hold entry A's sums, lanes 16-31 entry B's.
+__device__ __forceinline__ int sum_index(int lane) {
+  const bool b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
+  if (b0 && b1) return -1;
+  if (!b2) return (b3 ? 5 : 0) + (b0 ? 4 : b1 ? 2 : 0);
+  return b0 ? (b3 ? 10 : -1) : (b3 ? 5 : 0) + (b1 ? 3 : 1);
 }
 
-// Sums a warp's LaneSums into the eleven accumulators of a slot. A warp's lanes
-// are 4 row groups (lane >> 3) of 8 columns (lane & 7). dx is constant in a
-// column, so the rows are summed first (7 values, transposed so that each row
-// group is left with 1 to 3 of them) and only then multiplied by dx and dx^2;
-// the up to three values per group are then summed over the columns, again
-// transposed. 11 shuffles; 12 were needed for ten values formed per pixel.
-__device__ __forceinline__ float warp_reduce_moments(const LaneSums& v, float dx, float touched,
-                                                     int lane) {
-  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
-  // rows, 16 apart: groups 0, 1 take the moments, groups 2, 3 the rest
-  const float x0 = (b4 ? v.ab : v.a0) + __shfl_xor_sync(kFull, b4 ? v.a0 : v.ab, 16);
-  const float x1 = (b4 ? v.c0 : v.a1) + __shfl_xor_sync(kFull, b4 ? v.a1 : v.c0, 16);
-  const float x2 = (b4 ? v.c1 : v.a2) + __shfl_xor_sync(kFull, b4 ? v.a2 : v.c1, 16);
-  // (the moments have three values to the rest's four: groups 0, 1 get no x3)
-  const float x3 = v.c2 + __shfl_xor_sync(kFull, v.c2, 16);
-  // rows, 8 apart: groups 0 and 2 keep x0, groups 1 and 3 keep x1..x3
-  const float k0 = (b3 ? x1 : x0) + __shfl_xor_sync(kFull, b3 ? x0 : x1, 8);
-  const float k1 = x2 + __shfl_xor_sync(kFull, x2, 8);
-  const float k2 = x3 + __shfl_xor_sync(kFull, x3, 8);
-  // per column: group 0 a0 (1, dx, dx^2); group 1 a1 (1, dx), a2; group 2
-  // |dmean|, the touched flag (counted once); group 3 the colour
-  const float m = k0 * dx;
-  float o1 = b4 ? k1 : m;
-  float o2 = b4 ? k2 : (b3 ? k1 : m * dx);
-  if (b4 && !b3) o1 = (lane & 7) == 0 ? touched : 0.f;
-  // columns, 4 apart: the lower four lanes keep the first, the upper the others
-  const float p0 = (b2 ? o1 : k0) + __shfl_xor_sync(kFull, b2 ? k0 : o1, 4);
-  const float p1 = o2 + __shfl_xor_sync(kFull, o2, 4);
-  // columns, 2 apart: the upper four lanes split their two
-  const float r = ((b2 && b1) ? p1 : p0) + __shfl_xor_sync(kFull, (b2 && !b1) ? p1 : p0, 2);
-  return r + __shfl_xor_sync(kFull, r, 1);
+// Sums a warp's LaneSums of two entries A and B into the eleven accumulators of
+// each one's slot. The halves of the warp take one entry each, then lanes 8, 4,
+// 2 and 1 apart split what is left of its ten sums: 21 shuffles for the two
+// entries, against 24 for one reduction of ten values each, in the latency of
+// one. The touched flags need no sum; lane 13 of each half carries them.
+__device__ __forceinline__ float warp_reduce(const LaneSums& a, float toucheda,
+                                             const LaneSums& b, float touchedb, int lane) {
+  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
+  auto split = [&](bool upper, int apart, float x, float y) {
+    return (upper ? y : x) + __shfl_xor_sync(kFull, upper ? x : y, apart);
+  };
+  auto half = [&](float x, float y) { return split(b4, 16, x, y); };
+  // accumulators 0-4 to the lanes without bit 3, 5-9 to those with it
+  const float x0 = split(b3, 8, half(a.z, b.z), half(a.w, b.w));
+  const float x1 = split(b3, 8, half(a.uu, b.uu), half(a.c0, b.c0));
+  const float x2 = split(b3, 8, half(a.uw, b.uw), half(a.c1, b.c1));
+  const float x3 = split(b3, 8, half(a.ww, b.ww), half(a.c2, b.c2));
+  const float x4 = split(b3, 8, half(a.u, b.u), half(a.ab, b.ab));
+  const float y0 = split(b2, 4, x0, x1), y1 = split(b2, 4, x2, x3);
+  const float y2 = x4 + __shfl_xor_sync(kFull, x4, 4);
+  const float r0 = split(b1, 2, y0, y1), r1 = y2 + __shfl_xor_sync(kFull, y2, 2);
+  const float t = split(b0, 1, r0, r1);
+  return (lane & 15) == 13 ? (b4 ? touchedb : toucheda) : t;
 }
 
-// One entry's sums into its slot's accumulators, by the whole warp. `index` is
-// the lane's moment_index. (Entries that a single lane takes once had a path
-// of their own, without the reduction; finding them cost more than it saved:
-// adjoint 5.02 -> 4.91 ms per step of 8 views of 1920x1440, 1M gaussians, and
-// 3.00 -> 2.95 ms over 40 views of ten small scenes without it.)
-__device__ __forceinline__ void add_entry(ScreenGrad* slot, const LaneSums& v, float dx,
-                                          bool contrib, bool touched, int lane, int index) {
-  if (!__any_sync(kFull, contrib)) return;
+// Two entries' sums into their slots' accumulators, by the whole warp; `index`
+// is the lane's sum_index. (Entries that a single lane takes once had a path
+// of their own, without the reduction; finding them cost more than it saved.)
+__device__ __forceinline__ void add_entries(ScreenGrad* slot_a, const LaneSums& a, bool toucheda,
+                                            ScreenGrad* slot_b, const LaneSums& b, bool touchedb,
+                                            int lane, int index) {
+  const float any_a = __any_sync(kFull, toucheda) ? 1.f : 0.f;
+  const float any_b = __any_sync(kFull, touchedb) ? 1.f : 0.f;
+  const float sum = warp_reduce(a, any_a, b, any_b, lane);
+  float* dst = reinterpret_cast<float*>(lane < 16 ? slot_a : slot_b);
+  if (index >= 0) red_add(dst + index, sum);
+}
+
+// The same for one entry.
+__device__ __forceinline__ void add_entry(ScreenGrad* slot, const LaneSums& v, bool touched,
+                                          int lane, int index) {
+  const LaneSums none = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const float any = __any_sync(kFull, touched) ? 1.f : 0.f;
-  const float sum = warp_reduce_moments(v, dx, any, lane);
-  if (index >= 0) red_add(reinterpret_cast<float*>(slot) + index, sum);
+  const float sum = warp_reduce(v, any, none, 0.f, lane);
+  if (index >= 0 && lane < 16) red_add(reinterpret_cast<float*>(slot) + index, sum);
 }
 
 }  // namespace
@@ -138,7 +137,7 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
     behind[p] = bg0 * dLp0[p] + bg1 * dLp1[p] + bg2 * dLp2[p];
     thread_hi = max(thread_hi, my_last[p]);
   }
-  const int lane = lane_id(), warp = warp_id(), index = moment_index(lane_id());
+  const int lane = lane_id(), warp = warp_id(), index = sum_index(lane_id());
   const int warp_hi = __reduce_max_sync(kFull, thread_hi);
   if (threadIdx.x == 0) s_hi = info.range.x;
   __syncthreads();
@@ -171,7 +170,7 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
       const float4 co = s_co[j];
       const float4 c = s_col[j];
       const float dx = fx - m.x;
-      LaneSums v = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      LaneSums v = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       bool contrib = false, touched = false;
 #pragma unroll
       for (int p = 0; p < PX; ++p) {
@@ -194,18 +193,22 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
               if (raw_alpha < kMaxAlpha) {  // the cap flattens the gradient
                 touched = true;
                 const float z = raw_alpha * (d * T[p]);
-                const float zy = z * dy;
-                v.a0 += z;
-                v.a1 += zy;
-                v.a2 += zy * dy;
                 const float u = co.x * dx + co.y * dy, w = co.y * dx + co.z * dy;
+                const float zu = z * u, zw = z * w;
+                v.z += z;
+                v.uu += zu * u;
+                v.uw += zu * w;
+                v.ww += zw * w;
+                v.u += zu;
+                v.w += zw;
                 v.ab += fabsf(z) * sqrt_approx_ftz(u * u + w * w);
               }
             }
           }
         }
       }
-      add_entry(&screen[s_slot[j]], v, dx, contrib, touched, lane, index);
+      if (__any_sync(kFull, contrib))
+        add_entry(&screen[s_slot[j]], v, touched, lane, index);
     }
   }
 }
@@ -234,18 +237,23 @@ __device__ __forceinline__ uint32_t mask_from_block_bits(uint32_t bits) {
 // per lane.
 //
 // The kernel is bound by instruction issue (77% of cycles over whole waves,
-// ALU pipe 56%, FMA 44%), so its cost is instructions per entry and warp.
-// Summing the moments of dL/dpower instead of the mean, conic and opacity
-// gradients (their constants applied once per slot by the parameter chain),
-// the colour behind as its product with dL/drgb, and the sums straight to
-// global memory (a shared-memory float addition is a compare-and-swap loop)
-// took about 208 instructions to 145: 7.02 -> 4.91 ms per step of 8 views of
-// 1920x1440 with 1M gaussians, 4.18 -> 2.95 ms over 40 views of ten small
-// scenes, 0.131 -> 0.088 ms for one 320x240 view.
+// ALU pipe 56%, FMA 44%), so its cost is instructions per entry and warp, about
+// 208 of them when ten gradients per pixel were formed, reduced entry by entry
+// and added with shared-memory atomics (a compare-and-swap loop for floats):
+//   - the conic and opacity factors once per slot (ScreenGrad), the colour
+//     behind as its product with dL/drgb, sums straight to global memory;
+//   - two entries per reduction, which also halves the reduction's latency
+//     where few warps hide it (small images).
+// 7.02 -> 4.69 ms per step of 8 views of 1920x1440 with 1M gaussians, 4.18 ->
+// 2.81 ms over 40 views of ten small scenes, 0.131 -> 0.072 ms for one 320x240
+// view of 20k. Summing z, z d, z d^T d instead (seven lane sums, dx applied
+// once per column) ran in 4.39 ms but lost precision in elongated splats
+// (ScreenGrad); 9 or 10 CTAs per SM (56 or 48 registers, spills) in 4.80 and
+// 4.73 ms.
 // kB entries are staged per batch (RasterConfig::backward_batch: 64, 128 or
 // 256 with two pixels per thread; 128 with four, where fewer threads share a
 // batch); `schedule` maps CTAs to tiles (for_each_tile).
-template <int NP, int kB>
+template <int NP, int kB, bool kBits>
 __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
     k_backward_pairs(const int2* __restrict__ ranges, const uint32_t* __restrict__ pair_slots,
                      const float2* __restrict__ xy, const float4* __restrict__ conic_op,
@@ -306,7 +314,7 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
                                       __fmul2_rn(make_float2(b0, b0), nL0[q])));
     hi_mine = max(hi_mine, max(last0[q], last1[q]));
   }
-  const int lane = lane_id(), warp = warp_id(), index = moment_index(lane_id());
+  const int lane = lane_id(), warp = warp_id(), index = sum_index(lane_id());
   const int warp_hi = __reduce_max_sync(kFull, hi_mine);
   if (threadIdx.x == 0) s_hi = info.range.x;
   __syncthreads();
@@ -328,7 +336,7 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
       s_col[i] = color[slot];
       // which warps took the entry in the forward pass (exact), else which
       // ones its footprint can reach
-      s_mask[i] = block_bits != nullptr
+      s_mask[i] = kBits
                       ? mask_from_block_bits<PX>(block_bits[batch_start + i])
                       : warp_mask<PX>(mean, co, power_floor(co.w, min_alpha), info.tile_px,
                                       info.tile_py);
@@ -346,15 +354,15 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
       n_mine += __popc(b);
     }
     __syncwarp();
-    for (int qi = n_mine - 1; qi >= 0; --qi) {  // back to front
-      const int j = s_list[warp][qi];
+    // entry j's sums over this lane's pixels; whether a pixel took it, and one
+    // below the cap
+    auto visit = [&](int j, LaneSums& v, bool& contrib, bool& touched) {
       const int e = batch_start + j;
       const float2 nm = s_xy[j];
       const float4 co = s_co[j];
       const float4 c = s_col[j];
       const float dx = fx + nm.x;
-      bool contrib = false, touched = false;
-      LaneSums v;
+      contrib = touched = false;
       // pair q's sums: assigned by the first pair, added by the next
       auto put = [&](int q, float& to, float x) { to = q == 0 ? x : to + x; };
       const float adx = co.x * dx, bdx = co.y * dx;
@@ -404,19 +412,41 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
         touched = touched || t0 || t1;
         const float2 z = __fmul2_rn(make_float2(t0 ? nr.x : 0.f, t1 ? nr.y : 0.f),
                                     __fmul2_rn(nd, T[q]));
-        const float2 zy = __fmul2_rn(z, dy);
-        const float2 zyy = __fmul2_rn(zy, dy);
-        put(q, v.a0, z.x + z.y);
-        put(q, v.a1, zy.x + zy.y);
-        put(q, v.a2, zyy.x + zyy.y);
-        // |dL/dmean| per pixel, |z| |A d|, for the densification statistic (a
-        // sum compared against a threshold): the square-root approximation
         const float2 u = __ffma2_rn(make_float2(co.y, co.y), dy, make_float2(adx, adx));
         const float2 w = __ffma2_rn(make_float2(co.z, co.z), dy, make_float2(bdx, bdx));
+        const float2 zu = __fmul2_rn(z, u), zw = __fmul2_rn(z, w);
+        const float2 zuu = __fmul2_rn(zu, u), zuw = __fmul2_rn(zu, w), zww = __fmul2_rn(zw, w);
+        put(q, v.z, z.x + z.y);
+        put(q, v.uu, zuu.x + zuu.y);
+        put(q, v.uw, zuw.x + zuw.y);
+        put(q, v.ww, zww.x + zww.y);
+        put(q, v.u, zu.x + zu.y);
+        put(q, v.w, zw.x + zw.y);
+        // |dL/dmean| per pixel, |z| |A d|, for the densification statistic (a
+        // sum compared against a threshold): the square-root approximation
         const float2 sq = __ffma2_rn(u, u, __fmul2_rn(w, w));
         put(q, v.ab, fabsf(z.x) * sqrt_approx_ftz(sq.x) + fabsf(z.y) * sqrt_approx_ftz(sq.y));
       }
-      add_entry(&screen[s_slot[j]], v, dx, contrib, touched, lane, index);
+    };
+    // back to front, two entries at a time (one reduction serves both), then
+    // the odd one
+    int qi = n_mine - 1;
+    for (; qi > 0; qi -= 2) {
+      const int ja = s_list[warp][qi], jb = s_list[warp][qi - 1];
+      LaneSums va, vb;
+      bool ca, cb, ta, tb;
+      visit(ja, va, ca, ta);
+      visit(jb, vb, cb, tb);
+      if (kBits || __any_sync(kFull, ca || cb))
+        add_entries(&screen[s_slot[ja]], va, ta, &screen[s_slot[jb]], vb, tb, lane, index);
+    }
+    if (qi == 0) {
+      const int j = s_list[warp][0];
+      LaneSums v;
+      bool contrib, touched;
+      visit(j, v, contrib, touched);
+      if (kBits || __any_sync(kFull, contrib))
+        add_entry(&screen[s_slot[j]], v, touched, lane, index);
     }
   }
   });
@@ -435,7 +465,7 @@ void backward_px(const int2* ranges, const uint32_t* pair_slots, const float2* x
 
 }  // namespace
 
-template <int NP, int B>
+template <int NP, int B, bool kBits>
 void backward_pairs_launch(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
                            const float4* conic_op, const float4* color, const ViewDesc* views,
                            int n_views, int total_tiles, const float* T_final,
@@ -445,10 +475,11 @@ void backward_pairs_launch(const int2* ranges, const uint32_t* pair_slots, const
   const int schedule = tile_order == nullptr ? kTileOrder : raster_config().backward_schedule;
   int grid = total_tiles;
   if (schedule == kPersistent) {
-    grid = std::min(total_tiles, resident_ctas(k_backward_pairs<NP, B>, TileGeom<2 * NP>::kThreads));
+    grid = std::min(total_tiles,
+                    resident_ctas(k_backward_pairs<NP, B, kBits>, TileGeom<2 * NP>::kThreads));
     cudaMemsetAsync(ticket, 0, sizeof(int), stream);
   }
-  k_backward_pairs<NP, B><<<grid, TileGeom<2 * NP>::kThreads, 0, stream>>>(
+  k_backward_pairs<NP, B, kBits><<<grid, TileGeom<2 * NP>::kThreads, 0, stream>>>(
       ranges, pair_slots, xy, conic_op, color, views, n_views, T_final, last, dL_drgb, screen,
       block_bits, schedule, tile_order, ticket, total_tiles);
 }
@@ -460,28 +491,30 @@ void launch_backward(const int2* ranges, const uint32_t* pair_slots, const float
                      const uint8_t* block_bits, const int* tile_order, int* ticket) {
   if (total_tiles <= 0) return;
   count_launch();
+#define PXS_BWD(NP, B)                                                                         \
+  (block_bits != nullptr                                                                       \
+       ? backward_pairs_launch<NP, B, true>(ranges, pair_slots, xy, conic_op, color, views,    \
+                                            n_views, total_tiles, T_final, last, dL_drgb,      \
+                                            screen, stream, block_bits, tile_order, ticket)    \
+       : backward_pairs_launch<NP, B, false>(ranges, pair_slots, xy, conic_op, color, views,   \
+                                             n_views, total_tiles, T_final, last, dL_drgb,     \
+                                             screen, stream, block_bits, tile_order, ticket))
   switch (raster_config().backward_px) {
     case 1:
       backward_px<1>(ranges, pair_slots, xy, conic_op, color, views, n_views, total_tiles,
                      T_final, last, dL_drgb, screen, stream);
       break;
     case 4:
-      backward_pairs_launch<2, kBatch / 2>(ranges, pair_slots, xy, conic_op, color, views,
-                                           n_views, total_tiles, T_final, last, dL_drgb,
-                                           screen, stream, block_bits, tile_order, ticket);
+      PXS_BWD(2, kBatch / 2);
       break;
     default: {
       const int b = raster_config().backward_batch;
-#define PXS_BWD(B)                                                                         \
-  backward_pairs_launch<1, B>(ranges, pair_slots, xy, conic_op, color, views, n_views,    \
-                              total_tiles, T_final, last, dL_drgb, screen, stream, block_bits, \
-                              tile_order, ticket)
-      if (b == 64) PXS_BWD(64);
-      else if (b == 128) PXS_BWD(128);
-      else PXS_BWD(256);
-#undef PXS_BWD
+      if (b == 64) PXS_BWD(1, 64);
+      else if (b == 128) PXS_BWD(1, 128);
+      else PXS_BWD(1, 256);
     }
   }
+#undef PXS_BWD
 }
 
 }  // namespace pxs

@@ -1,11 +1,11 @@
 // adam.cu -- the optimiser step, fused with clearing the gradients and with
 // folding this step's densification statistics into the running totals.
 //
-// applyGradients (SplatTrainer.cpp:218-256) with adamDelta (:56-65), one
-// thread per gaussian so the quaternion can be renormalised in registers.
-// Compiled with -fmad=false: with IEEE division and square root the update is
-// bit-identical to the reference's for identical gradients.
-#include <tuple>
+// applyGradients (SplatTrainer.cpp:218-256) with adamDelta (:56-65). Compiled
+// with -fmad=false: with IEEE division and square root the update is bit-identical
+// to the reference's for identical gradients.
+#include <algorithm>
+#include <limits>
 #include <type_traits>
 
 #include "common.cuh"
@@ -13,263 +13,220 @@
 
 namespace pxs {
 
+// `plain`: every scalar is finite and epsilon and the corrections are positive.
+// Then a parameter that has never had a gradient (m = v = 0) moves by -lr 0 /
+// (0 + epsilon) = -0, which is left out: the divisions of 0 by a correction
+// would leave the fast path of IEEE division, and in a step that sees part of
+// the cloud most parameters are such (with their clearing 0.449 -> 0.296 ms at 1M
+// gaussians, 8 views; 0.119 -> 0.051 ms at 151,721, one view).
 __device__ __forceinline__ float adam_delta(float& m, float& v, float g, float lr, float b1,
-                                            float b2, float eps, float c1, float c2) {
+                                            float b2, float eps, float c1, float c2,
+                                            bool plain) {
   m = b1 * m + (1.f - b1) * g;
   v = b2 * v + (1.f - b2) * g * g;
-  const float m_hat = m / c1;
-  const float v_hat = v / c2;
-  return -lr * m_hat / (sqrtf(v_hat) + eps);
+  const bool still = plain && m == 0.f && v == 0.f;
+  const float m_hat = (still ? 1.f : m) / c1;
+  const float v_hat = (still ? 1.f : v) / c2;
+  const float delta = -lr * m_hat / (sqrtf(v_hat) + eps);
+  return still ? -m : delta;
 }
 
-__global__ void __launch_bounds__(256, 4)
+__device__ __forceinline__ bool plain_scalars(const StepScalars& s) {
+  const float rates = fabsf(s.lr[0]) + fabsf(s.lr[1]) + fabsf(s.lr[2]) + fabsf(s.lr[3]) +
+                      fabsf(s.lr[4]) + fabsf(s.lr[5]);
+  return s.epsilon > 0.f && s.correction1 > 0.f && s.correction2 > 0.f && isfinite(rates) &&
+         isfinite(s.epsilon) && isfinite(s.correction1) && isfinite(s.correction2);
+}
+
+// The groups of V floats of the flat P x N arrays (k_adam). The rows' sections
+// end at floats 3N, 6N, 10N, 11N, 14N and P N: the first group that begins at
+// or past each end, and the group that straddles it (the largest Index: none).
+// 32 bits count the groups of four of any arrays that fit the device.
+template <int V>
+struct AdamGroups {
+  using Index = std::conditional_t<V == 4, uint32_t, int64_t>;
+  Index next[6];
+  Index odd[6];
+  Index skipped;  // groups wholly inside the rotation rows
+};
+
+constexpr int kAdamThreads = 256, kAdamCtas = 6;
+
+// One kernel for every count and alignment. The parameters outside the rotation
+// are one elementwise problem: the flat P x N arrays are cut into groups of V
+// consecutive floats (V = 4, 16-byte loads and stores, where the arrays start
+// on 16 bytes, whatever N is: groups run across rows), one group per thread,
+// blocks [rot_blocks, grid). Blocks [0, rot_blocks) take a gaussian per thread:
+// its four rotation rows together, so the quaternion is renormalised in
+// registers, and its densify statistics. A group that straddles the rotation
+// rows' ends, or the array's, goes element by element.
+//
+// Bound by HBM: 28 bytes per float (32 when it clears the gradients), with about
+// 70 instructions per float of IEEE divisions and square root that keep the
+// reference's bits; 40 registers (6 CTAs per SM, a few bytes spilled around the
+// divisions' slow path) measured best. 333,333 gaussians SH3: 134.5 -> 102.3 us
+// (5.4 TB/s; rows of a count that is not a multiple of 4 took a gaussian per
+// thread before), 1M: 273.7 -> 266.2 us (6.2 TB/s).
+template <int V>
+__global__ void __launch_bounds__(kAdamThreads, kAdamCtas)
     k_adam(float* __restrict__ params, float* __restrict__ grads, float* __restrict__ m,
            float* __restrict__ v, int N, int S, const StepScalars* __restrict__ scalars,
            int zero_grads, float* __restrict__ screen_gradient,
            int32_t* __restrict__ visible_count, float* __restrict__ acc_gradient,
            int32_t* __restrict__ acc_views, const int32_t* __restrict__ skip,
-           const float* __restrict__ position_scale) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= N) return;
+           const float* __restrict__ position_scale, int rot_blocks, AdamGroups<V> groups) {
   // a step whose tile pairs overflowed is redone by the host: leave the state alone
   if (skip != nullptr && *skip != 0) return;
   const StepScalars& s = *scalars;
   const int64_t n = N;
-  const int P = 14 + 3 * S;
-  // positionLearningRate (SplatTrainer.cpp:200-208) ends with "* extent": with
-  // several scenes lr[0] holds the rest and each gaussian its scene's extent
-  const float lr_position = position_scale != nullptr ? s.lr[0] * position_scale[g] : s.lr[0];
-  // channels [c0, c0 + K) with learning rate lr(c): every load of the group
-  // is issued before its first store, so K channels' loads are in flight at once
-  auto update = [&](auto K, int c0, auto lr_of) {
-    constexpr int k = decltype(K)::value;
-    float pp[k], gg[k], mm[k], vv[k];
-#pragma unroll
-    for (int j = 0; j < k; ++j) {
-      const int64_t i = (int64_t)(c0 + j) * n + g;
-      pp[j] = params[i];
-      gg[j] = grads[i];
-      mm[j] = m[i];
-      vv[j] = v[i];
-    }
-#pragma unroll
-    for (int j = 0; j < k; ++j) {
-      const int64_t i = (int64_t)(c0 + j) * n + g;
-      params[i] = pp[j] + adam_delta(mm[j], vv[j], gg[j], lr_of(c0 + j), s.beta1, s.beta2,
-                                     s.epsilon, s.correction1, s.correction2);
-      m[i] = mm[j];
-      v[i] = vv[j];
-      if (zero_grads) grads[i] = 0.f;
-    }
-  };
-  using Six = std::integral_constant<int, 6>;
-  using Four = std::integral_constant<int, 4>;
-  using One = std::integral_constant<int, 1>;
-  // position and log-scale, then opacity and dc, then the SH rest
-  update(Six{}, 0, [&](int c) { return c < 3 ? lr_position : s.lr[1]; });
-  update(Four{}, PXS_C_OPACITY, [&](int c) { return c == PXS_C_OPACITY ? s.lr[3] : s.lr[4]; });
-  int c = PXS_C_SH_REST;
-  for (; c + 4 <= P; c += 4) update(Four{}, c, [&](int) { return s.lr[5]; });
-  for (; c < P; ++c) update(One{}, c, [&](int) { return s.lr[5]; });
-  float q[4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int64_t i = (int64_t)(PXS_C_ROTATION + a) * n + g;
-    float mm = m[i], vv = v[i];
-    q[a] = params[i] + adam_delta(mm, vv, grads[i], s.lr[2], s.beta1, s.beta2, s.epsilon,
-                                  s.correction1, s.correction2);
-    m[i] = mm;
-    v[i] = vv;
-    if (zero_grads) grads[i] = 0.f;
-  }
-  // Quaternion::norm / normalize over (x, y, z, w) storage (SplatTrainer.cpp:247-248)
-  const float sq = (q[1] * q[1] + q[3] * q[3]) + (q[2] * q[2] + q[0] * q[0]);
-  const float norm = sqrtf(sq);
-  if (norm > 1e-6f) {
-#pragma unroll
-    for (int a = 0; a < 4; ++a) q[a] = q[a] / norm;
-  } else {
-    q[0] = 1.f;
-    q[1] = q[2] = q[3] = 0.f;
-  }
-#pragma unroll
-  for (int a = 0; a < 4; ++a) params[(int64_t)(PXS_C_ROTATION + a) * n + g] = q[a];
-  // accumulateStatistics (SplatTrainer.cpp:258-263), then this step's stats clear
-  if (screen_gradient != nullptr) {
-    if (acc_gradient != nullptr) {
-      acc_gradient[g] += screen_gradient[g];
-      acc_views[g] += visible_count[g];
-    }
-    if (zero_grads) {
-      screen_gradient[g] = 0.f;
-      visible_count[g] = 0;
-    }
-  }
-}
-
-// Adam as an elementwise pass over (task, group of four gaussians), for N a
-// multiple of 4 (every component row then starts on a 16-byte boundary): a
-// thread updates one parameter row of four consecutive gaussians with 16-byte
-// loads and stores. Task t < 6 is row t (position, log-scale); task 6 is the
-// four rotation rows together, so the quaternion is renormalised in
-// registers; tasks 7.. are rows 10.. (opacity, dc, sh_rest); with statistics
-// the last task folds this step's densify statistics into the running totals.
-// Element by element the arithmetic of k_adam, so the results are the same
-// bits; many small independent threads keep enough loads in flight to stream
-// the eight P x N arrays at close to the memory bandwidth.
-__device__ __forceinline__ void ld4(const float* base, int64_t row, int64_t n, int g4,
-                                    float (&x)[4]) {
-  const float4 t = reinterpret_cast<const float4*>(base + row * n)[g4];
-  x[0] = t.x;
-  x[1] = t.y;
-  x[2] = t.z;
-  x[3] = t.w;
-}
-__device__ __forceinline__ void st4(float* base, int64_t row, int64_t n, int g4,
-                                    const float (&x)[4]) {
-  reinterpret_cast<float4*>(base + row * n)[g4] = make_float4(x[0], x[1], x[2], x[3]);
-}
-
-__global__ void __launch_bounds__(256)
-    k_adam_rows(float* __restrict__ params, float* __restrict__ grads, float* __restrict__ m,
-                float* __restrict__ v, int N, int S, const StepScalars* __restrict__ scalars,
-                int zero_grads, float* __restrict__ screen_gradient,
-                int32_t* __restrict__ visible_count, float* __restrict__ acc_gradient,
-                int32_t* __restrict__ acc_views, const int32_t* __restrict__ skip,
-                const float* __restrict__ position_scale) {
-  const int g4 = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g4 >= N / 4) return;
-  if (skip != nullptr && *skip != 0) return;
-  const StepScalars& s = *scalars;
-  const int64_t n = N;
-  const int P = 14 + 3 * S;
-  const int task = blockIdx.y;
-  const float zero[4] = {0.f, 0.f, 0.f, 0.f};
-  if (task == 6) {
-    float q[4][4];
+  const bool plain = plain_scalars(s);
+  if ((int)blockIdx.x < rot_blocks) {
+    const int g = blockIdx.x * kAdamThreads + threadIdx.x;
+    if (g >= N) return;
+    float q[4], gg[4], mm[4], vv[4];
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-      float pp[4], gg[4], mm[4], vv[4];
-      ld4(params, PXS_C_ROTATION + a, n, g4, pp);
-      ld4(grads, PXS_C_ROTATION + a, n, g4, gg);
-      ld4(m, PXS_C_ROTATION + a, n, g4, mm);
-      ld4(v, PXS_C_ROTATION + a, n, g4, vv);
+      const int64_t i = (PXS_C_ROTATION + a) * n + g;
+      q[a] = params[i];
+      gg[a] = grads[i];
+      mm[a] = m[i];
+      vv[a] = v[i];
+    }
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        q[a][e] = pp[e] + adam_delta(mm[e], vv[e], gg[e], s.lr[2], s.beta1, s.beta2, s.epsilon,
-                                     s.correction1, s.correction2);
-      st4(m, PXS_C_ROTATION + a, n, g4, mm);
-      st4(v, PXS_C_ROTATION + a, n, g4, vv);
-      if (zero_grads) st4(grads, PXS_C_ROTATION + a, n, g4, zero);
+    for (int a = 0; a < 4; ++a) {
+      const int64_t i = (PXS_C_ROTATION + a) * n + g;
+      q[a] = q[a] + adam_delta(mm[a], vv[a], gg[a], s.lr[2], s.beta1, s.beta2, s.epsilon,
+                               s.correction1, s.correction2, plain);
+      m[i] = mm[a];
+      v[i] = vv[a];
+      if (zero_grads) grads[i] = 0.f;
     }
     // Quaternion::norm / normalize over (x, y, z, w) storage (SplatTrainer.cpp:247-248)
+    const float sq = (q[1] * q[1] + q[3] * q[3]) + (q[2] * q[2] + q[0] * q[0]);
+    const float norm = sqrtf(sq);
+    if (norm > 1e-6f) {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float w = q[0][e], x = q[1][e], y = q[2][e], z = q[3][e];
-      const float sq = (x * x + z * z) + (y * y + w * w);
-      const float norm = sqrtf(sq);
-      if (norm > 1e-6f) {
+      for (int a = 0; a < 4; ++a) q[a] = q[a] / norm;
+    } else {
+      q[0] = 1.f;
+      q[1] = q[2] = q[3] = 0.f;
+    }
 #pragma unroll
-        for (int a = 0; a < 4; ++a) q[a][e] = q[a][e] / norm;
-      } else {
-        q[0][e] = 1.f;
-        q[1][e] = q[2][e] = q[3][e] = 0.f;
+    for (int a = 0; a < 4; ++a) params[(PXS_C_ROTATION + a) * n + g] = q[a];
+    // accumulateStatistics (SplatTrainer.cpp:258-263), then this step's stats clear
+    if (screen_gradient != nullptr) {
+      if (acc_gradient != nullptr) {
+        acc_gradient[g] += screen_gradient[g];
+        acc_views[g] += visible_count[g];
+      }
+      if (zero_grads) {
+        screen_gradient[g] = 0.f;
+        visible_count[g] = 0;
       }
     }
-#pragma unroll
-    for (int a = 0; a < 4; ++a) st4(params, PXS_C_ROTATION + a, n, g4, q[a]);
     return;
   }
-  const int row = task < 6 ? task : task + 3;  // tasks 7.. are rows 10..
-  if (row < P) {
-    float lr[4];
-    if (row < 3) {
-      float ps[4] = {1.f, 1.f, 1.f, 1.f};
-      if (position_scale != nullptr) ld4(position_scale, 0, n, g4, ps);
+  // group k: floats [k V, k V + V); the groups wholly inside the rotation rows
+  // are left out
+  using Index = typename AdamGroups<V>::Index;
+  Index k = (Index)(blockIdx.x - rot_blocks) * kAdamThreads + threadIdx.x;
+  if (k >= groups.next[1]) k += groups.skipped;
+  if (k >= groups.next[5]) return;
+  // positionLearningRate (SplatTrainer.cpp:200-208) ends with "* extent": with
+  // several scenes lr[0] holds the rest and each gaussian its scene's extent
+  const bool scaled = position_scale != nullptr && k < groups.next[0];
+  float lr = s.lr[5];
+  bool whole = V > 1 && k != groups.odd[5];
+  if (k < groups.next[4]) {
+    lr = k >= groups.next[3] ? s.lr[4]
+         : k >= groups.next[1] ? s.lr[3]
+         : k >= groups.next[0] ? s.lr[1]
+                               : s.lr[0];
+    whole = whole && !scaled && k != groups.odd[0] && k != groups.odd[1] &&
+            k != groups.odd[2] && k != groups.odd[3] && k != groups.odd[4];
+  }
+  if (whole) {
+    const float4 p4 = reinterpret_cast<const float4*>(params)[k];
+    const float4 g4 = reinterpret_cast<const float4*>(grads)[k];
+    const float4 m4 = reinterpret_cast<const float4*>(m)[k];
+    const float4 v4 = reinterpret_cast<const float4*>(v)[k];
+    float pp[4] = {p4.x, p4.y, p4.z, p4.w}, gg[4] = {g4.x, g4.y, g4.z, g4.w};
+    float mm[4] = {m4.x, m4.y, m4.z, m4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-      for (int e = 0; e < 4; ++e) lr[e] = position_scale != nullptr ? s.lr[0] * ps[e] : s.lr[0];
-    } else {
-      const float r = row < PXS_C_ROTATION ? s.lr[1]
-                      : row == PXS_C_OPACITY ? s.lr[3]
-                      : row < PXS_C_SH_REST  ? s.lr[4]
-                                             : s.lr[5];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) lr[e] = r;
-    }
-    float pp[4], gg[4], mm[4], vv[4];
-    ld4(params, row, n, g4, pp);
-    ld4(grads, row, n, g4, gg);
-    ld4(m, row, n, g4, mm);
-    ld4(v, row, n, g4, vv);
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      pp[e] += adam_delta(mm[e], vv[e], gg[e], lr[e], s.beta1, s.beta2, s.epsilon,
-                          s.correction1, s.correction2);
-    st4(params, row, n, g4, pp);
-    st4(m, row, n, g4, mm);
-    st4(v, row, n, g4, vv);
-    if (zero_grads) st4(grads, row, n, g4, zero);
+    for (int j = 0; j < 4; ++j)
+      pp[j] += adam_delta(mm[j], vv[j], gg[j], lr, s.beta1, s.beta2, s.epsilon, s.correction1,
+                          s.correction2, plain);
+    reinterpret_cast<float4*>(params)[k] = make_float4(pp[0], pp[1], pp[2], pp[3]);
+    reinterpret_cast<float4*>(m)[k] = make_float4(mm[0], mm[1], mm[2], mm[3]);
+    reinterpret_cast<float4*>(v)[k] = make_float4(vv[0], vv[1], vv[2], vv[3]);
+    if (zero_grads) reinterpret_cast<float4*>(grads)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     return;
   }
-  // accumulateStatistics (SplatTrainer.cpp:258-263), then this step's stats clear
-  if (screen_gradient != nullptr) {
-    float4* sg = reinterpret_cast<float4*>(screen_gradient);
-    int4* vc = reinterpret_cast<int4*>(visible_count);
-    if (acc_gradient != nullptr) {
-      float4 a4 = reinterpret_cast<float4*>(acc_gradient)[g4];
-      const float4 b = sg[g4];
-      a4.x += b.x;
-      a4.y += b.y;
-      a4.z += b.z;
-      a4.w += b.w;
-      reinterpret_cast<float4*>(acc_gradient)[g4] = a4;
-      int4 av = reinterpret_cast<int4*>(acc_views)[g4];
-      const int4 bv = vc[g4];
-      av.x += bv.x;
-      av.y += bv.y;
-      av.z += bv.z;
-      av.w += bv.w;
-      reinterpret_cast<int4*>(acc_views)[g4] = av;
-    }
-    if (zero_grads) {
-      sg[g4] = make_float4(0.f, 0.f, 0.f, 0.f);
-      vc[g4] = make_int4(0, 0, 0, 0);
-    }
+#pragma unroll 1
+  for (int j = 0; j < V; ++j) {
+    const int64_t e = (int64_t)k * V + j;
+    const int row = (int)(e / n);
+    if (row >= 14 + 3 * S) return;
+    if (row >= PXS_C_ROTATION && row < PXS_C_OPACITY) continue;
+    float rate = row < PXS_C_LOG_SCALE ? s.lr[0]
+                 : row < PXS_C_ROTATION ? s.lr[1]
+                 : row == PXS_C_OPACITY ? s.lr[3]
+                 : row < PXS_C_SH_REST  ? s.lr[4]
+                                        : s.lr[5];
+    if (row < PXS_C_LOG_SCALE && position_scale != nullptr) rate *= position_scale[e - row * n];
+    float mm = m[e], vv = v[e];
+    params[e] += adam_delta(mm, vv, grads[e], rate, s.beta1, s.beta2, s.epsilon, s.correction1,
+                            s.correction2, plain);
+    m[e] = mm;
+    v[e] = vv;
+    if (zero_grads) grads[e] = 0.f;
   }
 }
 
-// The elementwise form where every row (and every statistics array) is
-// 16-byte aligned, else one gaussian per thread.
-template <typename... A>
-void launch_adam_kernel(int N, const float* params, const float* grads, const float* screen,
-                        const int32_t* visible, const float* acc_gradient,
-                        const int32_t* acc_views, const float* position_scale,
-                        cudaStream_t stream, A... args) {
-  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-  const bool wide = N % 4 == 0 && aligned(params) && aligned(grads) &&
-                    (screen == nullptr || (aligned(screen) && aligned(visible))) &&
-                    (acc_gradient == nullptr || (aligned(acc_gradient) && aligned(acc_views))) &&
-                    (position_scale == nullptr || aligned(position_scale));
-  count_launch();
-  if (wide) {
-    // tasks: rows 0-5, the rotation rows, rows 10..P-1, the statistics
-    const int S = std::get<5>(std::make_tuple(args...));
-    const int tasks = 6 + 1 + (14 + 3 * S - 10) + (screen != nullptr ? 1 : 0);
-    k_adam_rows<<<dim3((N / 4 + 255) / 256, tasks), 256, 0, stream>>>(args...);
-  } else {
-    k_adam<<<(N + 255) / 256, 256, 0, stream>>>(args...);
+namespace {
+
+template <int V>
+void launch_adam_groups(float* params, float* grads, float* m, float* v, int N, int S,
+                        const StepScalars* scalars, int zero_grads, float* screen_gradient,
+                        int32_t* visible_count, float* acc_gradient, int32_t* acc_views,
+                        const int32_t* skip, cudaStream_t stream, const float* position_scale) {
+  using Index = typename AdamGroups<V>::Index;
+  const int64_t ends[6] = {3, 6, 10, 11, 14, 14 + 3 * (int64_t)S};  // rows
+  AdamGroups<V> groups;
+  for (int i = 0; i < 6; ++i) {
+    const int64_t end = ends[i] * N;
+    groups.next[i] = (Index)((end + V - 1) / V);
+    groups.odd[i] = end % V != 0 ? (Index)(end / V) : std::numeric_limits<Index>::max();
   }
+  groups.skipped = (Index)std::max<int64_t>(ends[2] * N / V - (int64_t)groups.next[1], 0);
+  const int rot_blocks = (N + kAdamThreads - 1) / kAdamThreads;
+  const int64_t blocks = rot_blocks + ((int64_t)groups.next[5] - (int64_t)groups.skipped +
+                                       kAdamThreads - 1) / kAdamThreads;
+  count_launch();
+  k_adam<V><<<(unsigned)blocks, kAdamThreads, 0, stream>>>(
+      params, grads, m, v, N, S, scalars, zero_grads, screen_gradient, visible_count,
+      acc_gradient, acc_views, skip, position_scale, rot_blocks, groups);
 }
+
+template <typename... Args>
+void launch_adam_kernel(float* params, float* grads, float* m, float* v, Args... args) {
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (aligned(params) && aligned(grads) && aligned(m) && aligned(v))
+    launch_adam_groups<4>(params, grads, m, v, args...);
+  else
+    launch_adam_groups<1>(params, grads, m, v, args...);
+}
+
+}  // namespace
 
 void launch_adam(float* params, float* grads, float* m, float* v, int N, int S,
                  const StepScalars* scalars, int zero_grads, float* screen_gradient,
                  int32_t* visible_count, float* acc_gradient, int32_t* acc_views,
                  cudaStream_t stream, const float* position_scale) {
   if (N <= 0) return;
-  launch_adam_kernel(N, params, grads, screen_gradient, visible_count, acc_gradient, acc_views,
-                     position_scale, stream, params, grads, m, v, N, S, scalars, zero_grads,
-                     screen_gradient, visible_count, acc_gradient, acc_views,
-                     static_cast<const int32_t*>(nullptr), position_scale);
+  launch_adam_kernel(params, grads, m, v, N, S, scalars, zero_grads, screen_gradient,
+                     visible_count, acc_gradient, acc_views, static_cast<const int32_t*>(nullptr),
+                     stream, position_scale);
 }
 
 void launch_adam_checked(float* params, float* grads, float* m, float* v, int N, int S,
@@ -278,10 +235,8 @@ void launch_adam_checked(float* params, float* grads, float* m, float* v, int N,
                          const int32_t* skip, cudaStream_t stream,
                          const float* position_scale) {
   if (N <= 0) return;
-  launch_adam_kernel(N, params, grads, screen_gradient, visible_count, acc_gradient, acc_views,
-                     position_scale, stream, params, grads, m, v, N, S, scalars, 1,
-                     screen_gradient, visible_count, acc_gradient, acc_views, skip,
-                     position_scale);
+  launch_adam_kernel(params, grads, m, v, N, S, scalars, 1, screen_gradient, visible_count,
+                     acc_gradient, acc_views, skip, stream, position_scale);
 }
 
 // resetOpacity (SplatTrainer.cpp:301-309): cap the logit, clear its moments.

@@ -438,7 +438,8 @@ int pxs_trainer_set_timing(pxs_trainer* trainer, int32_t enable);
 int pxs_trainer_stage_times(pxs_trainer* trainer, float* ms, int32_t capacity,
                             int32_t* n_stages, int32_t* n_steps);
 
-/* Tile pairs and kernel launches of the last step. */
+/* Tile pairs (entries of the tile lists the step built: the tiles each splat can
+ * reach a pixel of) and kernel launches of the last step. */
 int pxs_trainer_step_info(pxs_trainer* trainer, int64_t* pairs, int64_t* kernel_launches);
 
 /* Re-runs the last batch's forward pass counting the (pixel, entry) pairs the

@@ -82,7 +82,7 @@ pxs_raster_options default_options() {
 
 // Uploads a host cloud and runs projection and binning for one view.
 void render_setup(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* camera,
-                  const pxs_raster_options* options, bool debug_cov) {
+                  const pxs_raster_options* options, bool debug_cov, bool whole_lists = false) {
   validate_cloud(cloud);
   if (camera == nullptr) throw Error(PXS_ERR_INVALID, "camera is null");
   const pxs_raster_options opt = options ? *options : default_options();
@@ -94,7 +94,7 @@ void render_setup(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* ca
                              cudaMemcpyHostToDevice, ctx->stream));
   const pxs::ViewBatch batch = pxs::make_batch(camera, 1, opt, cloud->sh_degree);
   ctx->frame.prepare(batch, cloud->count, cloud->rest_per_channel, ctx->stream);
-  ctx->frame.project(d_params, ctx->stream, debug_cov);
+  ctx->frame.project(d_params, ctx->stream, debug_cov, whole_lists);
   ctx->frame.bin(true, ctx->stream);
 }
 
@@ -345,7 +345,7 @@ int pxs_tile_lists(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* c
   int status_capacity = PXS_OK;
   const int status = guarded(ctx, [&] {
     if (offsets == nullptr) throw Error(PXS_ERR_INVALID, "offsets is null");
-    render_setup(ctx, cloud, camera, options, false);
+    render_setup(ctx, cloud, camera, options, false, true);
     pxs::Frame& f = ctx->frame;
     const int tiles = f.batch.total_tiles;
     const int64_t K = f.last_pair_count;

@@ -77,7 +77,6 @@ struct ProjectedSoA {
   float4* color;       // r, g, b, clamp flags (bits in .w)
   uint32_t* depth_key; // float bits of depth; kCulledKey when culled
   uint2* rect;         // x0 | x1 << 16, y0 | y1 << 16 (tile coordinates)
-  int32_t* tile_count; // tiles touched
   float4* debug_cov;   // optional: cov2d (xx, xy, yy), radius
 };
 

@@ -30,8 +30,9 @@ struct ScanScratch {
 };
 
 // project.cu
+// `tight`: the tile rectangles cut to what a pixel can see of each splat.
 void launch_project(const float* params, int N, int S, int64_t slot_stride,
-                    const ViewDesc* views, int n_views, const ProjectedSoA& out,
+                    const ViewDesc* views, int n_views, const ProjectedSoA& out, bool tight,
                     cudaStream_t stream);
 void configure_param_grads_kernel();  // once per device, outside graph capture
 void launch_param_grads(const float* params, int N, int S, int64_t slot_stride,
@@ -69,8 +70,11 @@ void launch_slot_row_counts(const uint32_t* sorted_slots, const uint32_t* sorted
                             const uint2* rect, const ViewDesc* views, int n_views,
                             int64_t slot_stride, int max_tiles_y, int32_t* counts,
                             cudaStream_t stream);
+// `xy` and `conic_op` (both null for the whole rectangle): each record's columns
+// are cut to the ones its splat reaches in that row.
 void launch_slot_row_expand(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
-                            const uint2* rect, const ViewDesc* views, int n_views,
+                            const uint2* rect, const float2* xy, const float4* conic_op,
+                            const ViewDesc* views, int n_views,
                             int64_t slot_stride, int max_tiles_y, const int64_t* offsets,
                             int64_t capacity, uint32_t* rec_slots, uint32_t* rec_xr,
                             cudaStream_t stream);

@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "kernels.h"
 #include "project_common.cuh"
+#include "raster_common.cuh"
 
 namespace pxs {
 
@@ -26,7 +27,7 @@ constexpr int kProjectThreads = 256;
 template <int S>
 __global__ void __launch_bounds__(kProjectThreads, 3)
     k_project(const float* __restrict__ params, int N, int64_t slot_stride,
-              const ViewDesc* __restrict__ views, int n_views, ProjectedSoA out) {
+              const ViewDesc* __restrict__ views, int n_views, ProjectedSoA out, int tight) {
   constexpr int kRest = 3 * S > 0 ? 3 * S : 1;
   __shared__ float s_sh[kRest][kProjectThreads];
   const int t = threadIdx.x;
@@ -41,7 +42,6 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
     const ViewDesc& vd = views[v];
     if (i >= vd.gauss_count) {
       out.depth_key[slot] = kCulledKey;
-      out.tile_count[slot] = 0;
       continue;
     }
     if (vd.gauss_offset + i != g) {
@@ -104,7 +104,6 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
     }
     if (!visible) {
       out.depth_key[slot] = kCulledKey;
-      out.tile_count[slot] = 0;
       continue;
     }
     // evaluateSh (SplatRaster.cpp:179-199) along the unit camera->gaussian direction
@@ -144,20 +143,35 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
     out.depth_key[slot] = __float_as_uint(p[2]);
     if (out.debug_cov != nullptr)
       out.debug_cov[slot] = make_float4(cov[0], cov[1], cov[3], radius);
-    // tileRange (SplatRaster.cpp:121-126)
-    const int x0 = max(0, float_to_int_x86(floorf((mean_x - radius) / 16.f)));
-    const int x1 = min(vd.tiles_x - 1, float_to_int_x86(floorf((mean_x + radius) / 16.f)));
-    const int y0 = max(0, float_to_int_x86(floorf((mean_y - radius) / 16.f)));
-    const int y1 = min(vd.tiles_y - 1, float_to_int_x86(floorf((mean_y + radius) / 16.f)));
-    const int tiles = (x1 >= x0 && y1 >= y0) ? (x1 - x0 + 1) * (y1 - y0 + 1) : 0;
+    // tileRange (SplatRaster.cpp:121-126): the 3-sigma square. With `tight` it is
+    // cut to the tiles with a pixel the splat can reach (splat_footprint): an
+    // entry of any other tile passes no pixel's alpha test, so images and
+    // gradients are the same bits and the lists half as long.
+    int x0 = max(0, float_to_int_x86(floorf((mean_x - radius) / 16.f)));
+    int x1 = min(vd.tiles_x - 1, float_to_int_x86(floorf((mean_x + radius) / 16.f)));
+    int y0 = max(0, float_to_int_x86(floorf((mean_y - radius) / 16.f)));
+    int y1 = min(vd.tiles_y - 1, float_to_int_x86(floorf((mean_y + radius) / 16.f)));
+    if (tight) {
+      const Footprint f =
+          splat_footprint(make_float4(conic_a, conic_b, conic_c, st.opacity), vd.min_alpha);
+      if (!f.all) {
+        x0 = max(x0, first_tile(mean_x - f.ex));
+        x1 = min(x1, last_tile(mean_x + f.ex));
+        y0 = max(y0, first_tile(mean_y - f.ey));
+        y1 = min(y1, last_tile(mean_y + f.ey));
+        if (x0 > x1 || y0 > y1) {  // no rows, no columns
+          x0 = y0 = 1;
+          x1 = y1 = 0;
+        }
+      }
+    }
     out.rect[slot] = make_uint2((uint32_t)(x0 & 0xFFFF) | ((uint32_t)(x1 & 0xFFFF) << 16),
                                 (uint32_t)(y0 & 0xFFFF) | ((uint32_t)(y1 & 0xFFFF) << 16));
-    out.tile_count[slot] = tiles;
   }
 }
 
 void launch_project(const float* params, int N, int S, int64_t slot_stride,
-                    const ViewDesc* views, int n_views, const ProjectedSoA& out,
+                    const ViewDesc* views, int n_views, const ProjectedSoA& out, bool tight,
                     cudaStream_t stream) {
   const int threads = kProjectThreads;
   const int blocks = (int)((slot_stride + threads - 1) / threads);
@@ -165,16 +179,20 @@ void launch_project(const float* params, int N, int S, int64_t slot_stride,
   count_launch();
   switch (S) {
     case 0:
-      k_project<0><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out);
+      k_project<0><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out,
+                                                 tight);
       break;
     case 3:
-      k_project<3><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out);
+      k_project<3><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out,
+                                                 tight);
       break;
     case 8:
-      k_project<8><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out);
+      k_project<8><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out,
+                                                 tight);
       break;
     default:
-      k_project<15><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out);
+      k_project<15><<<blocks, threads, 0, stream>>>(params, N, slot_stride, views, n_views, out,
+                                                 tight);
       break;
   }
 }

@@ -281,4 +281,78 @@ __device__ __forceinline__ float power_floor(float opacity, float min_alpha) {
   return __logf(__fdividef(min_alpha, opacity)) - 1e-5f;
 }
 
+// The part of a splat that can reach a pixel: where power >= `floor`, i.e. the
+// ellipse q(d) = d^T A d <= k = -2 floor of its conic A, with the margins of
+// warp_mask: a conic with a c < 10 det ("mild") is taken at k (1 + 1e-4) + 1e-4
+// and padded by 0.02 px, which is ten times the rounding of its powers and of
+// these bounds; a more elongated one only by its box, widened by 10% and half a
+// pixel. `all` (no floor, no definite conic, extents of 1e4 px or not finite)
+// bounds nothing.
+struct Footprint {
+  float k, ex, ey, pad;
+  bool mild, all;
+};
+__device__ __forceinline__ Footprint splat_footprint(const float4& co, float min_alpha) {
+  Footprint f;
+  const float floor = power_floor(co.w, min_alpha);
+  const float det = co.x * co.z - co.y * co.y;
+  f.mild = co.x * co.z < 10.f * det;
+  f.k = -2.f * floor;
+  if (f.mild) f.k = f.k * 1.0001f + 1e-4f;
+  const float inv_det = __fdividef(1.f, det);
+  const float widen = f.mild ? 1.0001f : 1.1f;
+  f.pad = f.mild ? 0.02f : 0.5f;
+  f.ex = sqrt_approx(f.k * co.z * inv_det) * widen + f.pad;
+  f.ey = sqrt_approx(f.k * co.x * inv_det) * widen + f.pad;
+  f.all = !(floor > -1e30f) || !(det > 0.f) || !(f.ex < 1e4f && f.ey < 1e4f);
+  return f;
+}
+
+// First and last tile along an axis with a pixel centre in [lo, hi].
+__device__ __forceinline__ int first_tile(float lo) {
+  return __float2int_ru((lo - ((float)kTile - 0.5f)) * (1.f / kTile));
+}
+__device__ __forceinline__ int last_tile(float hi) {
+  return __float2int_rd((hi - 0.5f) * (1.f / kTile));
+}
+
+// What row_columns needs of a splat: mean, conic b and 1 / a, the dy of its
+// footprint's right end (the left end's is its negative), a k and the
+// determinant; ia = 0: nothing to cut.
+struct alignas(16) RowShape {
+  float mx, my, b, ia;
+  float end, ak, det;
+  uint32_t x;  // the tile columns of its box, x0 | x1 << 16
+};
+__device__ __forceinline__ RowShape row_shape(const Footprint& f, const float4& co, float2 mean,
+                                              uint32_t x) {
+  RowShape r;
+  r.mx = mean.x;
+  r.my = mean.y;
+  r.b = co.y;
+  r.x = x;
+  r.det = co.x * co.z - co.y * co.y;
+  r.ak = co.x * f.k;
+  r.end = __fdividef(-co.y, co.z) * sqrt_approx(__fdividef(f.k * co.z, r.det));
+  r.ia = f.all || !f.mild ? 0.f : __fdividef(1.f, co.x);
+  return r;
+}
+
+// The tile columns x0 | x1 << 16 of tile row `row` that a splat's footprint
+// reaches, of its box's (1: none, as 1 > 0). Across the row's band of pixel
+// centres the ellipse is widest at its own left and right end or at the band's
+// edge nearest to them.
+__device__ __forceinline__ uint32_t row_columns(const RowShape& r, int row) {
+  if (r.ia == 0.f) return r.x;
+  constexpr float kPad = 0.02f;  // splat_footprint's for these conics
+  const float lo = ((float)(row * kTile) + (0.5f - kPad)) - r.my;
+  const float hi = lo + ((float)(kTile - 1) + 2.f * kPad);
+  const float yr = fminf(fmaxf(r.end, lo), hi), yl = fminf(fmaxf(-r.end, lo), hi);
+  const float right = (sqrt_approx_ftz(fmaxf(r.ak - r.det * yr * yr, 0.f)) - r.b * yr) * r.ia;
+  const float left = -(sqrt_approx_ftz(fmaxf(r.ak - r.det * yl * yl, 0.f)) + r.b * yl) * r.ia;
+  const int x0 = max((int)(r.x & 0xFFFF), first_tile(r.mx + left - kPad));
+  const int x1 = min((int)(r.x >> 16), last_tile(r.mx + right + kPad));
+  return x0 <= x1 ? (uint32_t)x0 | ((uint32_t)x1 << 16) : 1u;
+}
+
 }  // namespace pxs

@@ -129,7 +129,6 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   color.reserve(slots);
   depth_key.reserve(slots);
   rect.reserve(slots);
-  tile_count.reserve(slots);
   sort_keys.reserve(slots);
   sort_vals.reserve(slots);
   sort_keys_alt.reserve(slots);
@@ -203,17 +202,18 @@ void Frame::ensure_chunks() {
   }
 }
 
-void Frame::project(const float* params, cudaStream_t stream, bool want_debug) {
+void Frame::project(const float* params, cudaStream_t stream, bool want_debug,
+                    bool whole_lists) {
+  whole_lists_ = whole_lists;
   ProjectedSoA out;
   out.xy = xy.get();
   out.conic_op = conic_op.get();
   out.color = color.get();
   out.depth_key = depth_key.get();
   out.rect = rect.get();
-  out.tile_count = tile_count.get();
   out.debug_cov = nullptr;
   if (want_debug) out.debug_cov = debug_cov.reserve(static_cast<size_t>(V) * slot_stride);
-  launch_project(params, N, S, slot_stride, d_views.get(), V, out, stream);
+  launch_project(params, N, S, slot_stride, d_views.get(), V, out, !whole_lists, stream);
   PXS_CUDA(cudaGetLastError());
 }
 
@@ -253,7 +253,8 @@ int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
     throw Error(PXS_ERR_INVALID, "pair buffers must be reserved before an unsynchronised bin");
   }
   PXS_CUDA(cudaMemsetAsync(overflow.get(), 0, sizeof(int32_t), stream));
-  launch_slot_row_expand(v, k, rect.get(), d_views.get(), V, slot_stride,
+  launch_slot_row_expand(v, k, rect.get(), whole_lists_ ? nullptr : xy.get(),
+                         whole_lists_ ? nullptr : conic_op.get(), d_views.get(), V, slot_stride,
                          batch.max_tiles_y, row_chunk_offsets.get(), record_capacity,
                          rec_vals.get(), rec_xr.get(), stream);
   launch_row_ranges_from_chunks(row_chunk_offsets.get(), batch.total_rows, cpv,

@@ -120,8 +120,11 @@ class Frame {
  public:
   // Sizes the per-slot and per-pixel buffers and uploads the views.
   void prepare(const ViewBatch& batch, int N, int S, cudaStream_t stream);
-  // Project every (view, gaussian) slot.
-  void project(const float* params, cudaStream_t stream, bool debug_cov = false);
+  // Project every (view, gaussian) slot. The tile lists that bin() then builds
+  // hold the tiles a splat can reach, or with `whole_lists` every tile of its
+  // 3-sigma square, as the reference's do.
+  void project(const float* params, cudaStream_t stream, bool debug_cov = false,
+               bool whole_lists = false);
   // Depth sort, pair emission, tile sort and ranges. With host_sync the pair
   // count is read back and the pair buffers grown to fit; otherwise the
   // preallocated capacity is used and an overflow raises the overflow flag.
@@ -153,7 +156,6 @@ class Frame {
   DeviceArray<float4> conic_op, color, debug_cov;
   DeviceArray<uint32_t> depth_key;
   DeviceArray<uint2> rect;
-  DeviceArray<int32_t> tile_count;
   DeviceArray<uint32_t> sort_keys, sort_vals, sort_keys_alt, sort_vals_alt;
   // per (tile row, chunk of depth-sorted slots): records and their offsets
   DeviceArray<int32_t> row_chunk_counts;
@@ -190,6 +192,7 @@ class Frame {
   uint32_t* sorted_slots = nullptr;
 
  private:
+  bool whole_lists_ = false;
   void ensure_scan_scratch(int64_t n);
   void ensure_chunks();
   ScanScratch scan_;

@@ -304,8 +304,7 @@ int pxs_project(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* came
     const size_t slots = static_cast<size_t>(f.slot_stride);
     const auto order = download(f.sorted_slots, slots, ctx->stream);
     const auto keys = download(f.depth_key.get(), slots, ctx->stream);
-    const auto xy = download(f.xy.get(), slots, ctx->stream);
-    const auto co = download(f.conic_op.get(), slots, ctx->stream);
+    const auto geom = download(f.geom.get(), slots, ctx->stream);
     const auto col = download(f.color.get(), slots, ctx->stream);
     const auto cov = download(f.debug_cov.get(), slots, ctx->stream);
     PXS_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -315,16 +314,16 @@ int pxs_project(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* came
       if (keys[s] == pxs::kCulledKey) break;
       pxs_projected_splat& p = out[n++];
       p.index = static_cast<int32_t>(s);
-      p.mean[0] = xy[s].x;
-      p.mean[1] = xy[s].y;
+      p.mean[0] = geom[s].xy.x;
+      p.mean[1] = geom[s].xy.y;
       p.cov2d[0] = cov[s].x;
       p.cov2d[1] = cov[s].y;
       p.cov2d[2] = cov[s].z;
       p.radius = cov[s].w;
-      p.conic[0] = co[s].x;
-      p.conic[1] = co[s].y;
-      p.conic[2] = co[s].z;
-      p.opacity = co[s].w;
+      p.conic[0] = geom[s].conic_op.x;
+      p.conic[1] = geom[s].conic_op.y;
+      p.conic[2] = geom[s].conic_op.z;
+      p.opacity = geom[s].conic_op.w;
       float depth;
       std::memcpy(&depth, &keys[s], sizeof(float));
       p.depth = depth;

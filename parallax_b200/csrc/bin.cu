@@ -448,7 +448,7 @@ constexpr int kSlotPerLane = kSlotChunk / (kWarps * 32);  // slots per lane per 
 // rectangle is never empty (its footprint meets the image).
 __device__ __forceinline__ void chunk_slot_rows(const uint32_t* __restrict__ sorted_slots,
                                                 const uint32_t* __restrict__ sorted_keys,
-                                                const uint2* __restrict__ rect, int64_t begin,
+                                                const SlotGeom* __restrict__ geom, int64_t begin,
                                                 uint32_t (&slot)[kSlotPerLane],
                                                 uint32_t (&yr)[kSlotPerLane],
                                                 uint32_t (*xr)[kSlotPerLane] = nullptr) {
@@ -465,7 +465,7 @@ __device__ __forceinline__ void chunk_slot_rows(const uint32_t* __restrict__ sor
 #pragma unroll
   for (int k = 0; k < kSlotPerLane; ++k)
     if (live[k]) {
-      const uint2 r = rect[slot[k]];
+      const uint2 r = geom[slot[k]].rect;
       yr[k] = r.y;
       if (xr != nullptr) (*xr)[k] = r.x;
     }
@@ -475,7 +475,8 @@ __device__ __forceinline__ void chunk_slot_rows(const uint32_t* __restrict__ sor
 // v * cpv + c) covering tile row y of the view.
 __global__ void __launch_bounds__(kWarps * 32)
     k_slot_row_counts(const uint32_t* __restrict__ sorted_slots,
-                      const uint32_t* __restrict__ sorted_keys, const uint2* __restrict__ rect,
+                      const uint32_t* __restrict__ sorted_keys,
+                      const SlotGeom* __restrict__ geom,
                       const ViewDesc* __restrict__ views, int64_t slot_stride, int cpv,
                       int max_tiles_y, int32_t* __restrict__ counts) {
   extern __shared__ int32_t s_cnt[];  // [kWarps][max_tiles_y]
@@ -486,7 +487,7 @@ __global__ void __launch_bounds__(kWarps * 32)
     s_cnt[(i / tiles_y) * max_tiles_y + (i % tiles_y)] = 0;
   __syncthreads();
   uint32_t slot[kSlotPerLane], yr[kSlotPerLane];
-  chunk_slot_rows(sorted_slots, sorted_keys, rect,
+  chunk_slot_rows(sorted_slots, sorted_keys, geom,
                   (int64_t)v * slot_stride + (int64_t)c * kSlotChunk, slot, yr);
   warp_range_counts(yr, tiles_y, s_cnt + warp_id() * max_tiles_y);
   __syncthreads();
@@ -500,8 +501,8 @@ __global__ void __launch_bounds__(kWarps * 32)
 
 // The chunk's records at offsets[(row_offset + y) * cpv + c] onwards in each
 // row y, in slot order; nothing at or past `capacity`. A record's columns are
-// cut to the ones its splat reaches in that row (row_columns; with xy null they
-// stay the rectangle's). That arithmetic runs on the staged records, a lane per
+// cut to the ones its splat reaches in that row (row_columns; without
+// `tight` they stay the rectangle's). That arithmetic runs on the staged records, a lane per
 // record with the row uniform, on shapes kept in shared memory: in the ranking
 // loop, where the lanes' splats have different numbers of rows, it was slower
 // (the kernel in 0.64 against 0.58 ms, 8 views of 1M gaussians
@@ -514,8 +515,8 @@ struct RowExpandSmem {
 
 __global__ void __launch_bounds__(kWarps * 32)
     k_slot_row_expand(const uint32_t* __restrict__ sorted_slots,
-                      const uint32_t* __restrict__ sorted_keys, const uint2* __restrict__ rect,
-                      const float2* __restrict__ xy, const float4* __restrict__ conic_op,
+                      const uint32_t* __restrict__ sorted_keys,
+                      const SlotGeom* __restrict__ geom, int tight,
                       const ViewDesc* __restrict__ views, int64_t slot_stride, int cpv,
                       int max_tiles_y, const int64_t* __restrict__ offsets, int64_t capacity,
                       uint32_t* __restrict__ rec_slots, uint32_t* __restrict__ rec_xr) {
@@ -535,7 +536,7 @@ __global__ void __launch_bounds__(kWarps * 32)
   }
   uint32_t slot[kSlotPerLane], yr[kSlotPerLane];
   uint32_t xr[kSlotPerLane];  // the box's column ranges
-  chunk_slot_rows(sorted_slots, sorted_keys, rect,
+  chunk_slot_rows(sorted_slots, sorted_keys, geom,
                   (int64_t)v * slot_stride + (int64_t)c * kSlotChunk, slot, yr, &xr);
   const int place = w * (kSlotChunk / kWarps) + lane;  // of the lane's first splat
 #pragma unroll
@@ -544,9 +545,10 @@ __global__ void __launch_bounds__(kWarps * 32)
     RowShape shape;
     shape.x = xr[k];
     shape.ia = 0.f;
-    if (xy != nullptr && (yr[k] >> 16) >= (yr[k] & 0xFFFF)) {
-      const float4 co = conic_op[slot[k]];
-      shape = row_shape(splat_footprint(co, vd.min_alpha), co, xy[slot[k]], xr[k]);
+    if (tight && (yr[k] >> 16) >= (yr[k] & 0xFFFF)) {
+      const float4 co = geom[slot[k]].conic_op;
+      const Footprint f = splat_footprint(co, vd.min_alpha);
+      shape = row_shape(f, co, geom[slot[k]].xy, xr[k]);
     }
     sm.shape[place + k * 32] = shape;
   }
@@ -645,19 +647,19 @@ void configure_bin_kernels() {
 int slot_chunks_per_view(int64_t slot_stride) { return (int)(slot_stride / kSlotChunk); }
 
 void launch_slot_row_counts(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
-                            const uint2* rect, const ViewDesc* views, int n_views,
+                            const SlotGeom* geom, const ViewDesc* views, int n_views,
                             int64_t slot_stride, int max_tiles_y, int32_t* counts,
                             cudaStream_t stream) {
   const int cpv = slot_chunks_per_view(slot_stride);
   if (n_views <= 0 || cpv <= 0) return;
   count_launch();
   k_slot_row_counts<<<(unsigned)(n_views * cpv), kWarps * 32, slot_row_counts_smem(max_tiles_y),
-                      stream>>>(sorted_slots, sorted_keys, rect, views, slot_stride, cpv,
+                      stream>>>(sorted_slots, sorted_keys, geom, views, slot_stride, cpv,
                                 max_tiles_y, counts);
 }
 
 void launch_slot_row_expand(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
-                            const uint2* rect, const float2* xy, const float4* conic_op,
+                            const SlotGeom* geom, bool tight,
                             const ViewDesc* views, int n_views,
                             int64_t slot_stride, int max_tiles_y, const int64_t* offsets,
                             int64_t capacity, uint32_t* rec_slots, uint32_t* rec_xr,
@@ -666,7 +668,7 @@ void launch_slot_row_expand(const uint32_t* sorted_slots, const uint32_t* sorted
   if (n_views <= 0 || cpv <= 0) return;
   count_launch();
   k_slot_row_expand<<<(unsigned)(n_views * cpv), kWarps * 32, slot_row_expand_smem(max_tiles_y),
-                      stream>>>(sorted_slots, sorted_keys, rect, xy, conic_op, views,
+                      stream>>>(sorted_slots, sorted_keys, geom, tight, views,
                                 slot_stride, cpv, max_tiles_y, offsets, capacity, rec_slots, rec_xr);
 }
 

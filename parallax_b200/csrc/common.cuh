@@ -70,13 +70,20 @@ struct alignas(16) ScreenGrad {
 };
 static_assert(sizeof(ScreenGrad) == 48, "ScreenGrad layout");
 
+// What a (view, gaussian) slot's projection leaves for binning, compositing and
+// its adjoint, which gather slots in depth order: one aligned 32-byte sector, so
+// that a gather costs one (as three arrays it cost up to three).
+struct alignas(32) SlotGeom {
+  float4 conic_op;  // conic (a, b, c), opacity
+  float2 xy;        // mean
+  uint2 rect;       // tile coordinates x0 | x1 << 16, y0 | y1 << 16
+};
+
 // Device views of the per-slot projection outputs.
 struct ProjectedSoA {
-  float2* xy;          // mean
-  float4* conic_op;    // conic (a, b, c), opacity
+  SlotGeom* geom;
   float4* color;       // r, g, b, clamp flags (bits in .w)
   uint32_t* depth_key; // float bits of depth; kCulledKey when culled
-  uint2* rect;         // x0 | x1 << 16, y0 | y1 << 16 (tile coordinates)
   float4* debug_cov;   // optional: cov2d (xx, xy, yy), radius
 };
 

@@ -37,7 +37,7 @@ void launch_project(const float* params, int N, int S, int64_t slot_stride,
 void configure_param_grads_kernel();  // once per device, outside graph capture
 void launch_param_grads(const float* params, int N, int S, int64_t slot_stride,
                         const ViewDesc* views, int n_views, const uint32_t* depth_key,
-                        const float4* conic_op, const float4* color, const ScreenGrad* screen,
+                        const SlotGeom* geom, const float4* color, const ScreenGrad* screen,
                         float* grads, float* screen_gradient, int32_t* visible_count,
                         cudaStream_t stream);
 
@@ -67,13 +67,12 @@ void configure_bin_kernels();  // once per device, outside graph capture
 // offsets, each chunk writes its records (slot ids) at its bases.
 int slot_chunks_per_view(int64_t slot_stride);
 void launch_slot_row_counts(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
-                            const uint2* rect, const ViewDesc* views, int n_views,
+                            const SlotGeom* geom, const ViewDesc* views, int n_views,
                             int64_t slot_stride, int max_tiles_y, int32_t* counts,
                             cudaStream_t stream);
-// `xy` and `conic_op` (both null for the whole rectangle): each record's columns
-// are cut to the ones its splat reaches in that row.
+// With `tight` each record's columns are cut to the ones its splat reaches in that row.
 void launch_slot_row_expand(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
-                            const uint2* rect, const float2* xy, const float4* conic_op,
+                            const SlotGeom* geom, bool tight,
                             const ViewDesc* views, int n_views,
                             int64_t slot_stride, int max_tiles_y, const int64_t* offsets,
                             int64_t capacity, uint32_t* rec_slots, uint32_t* rec_xr,
@@ -129,8 +128,7 @@ void launch_tile_order(const int2* ranges, int total_tiles, int* order, int* wor
 // writes, per tile-list entry, a byte whose bit b is set when some pixel of
 // the tile's 8x8 block b (b = 2 * row block + column block) took the entry.
 // Returns whether it wrote them.
-bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                    const float4* conic_op, const float4* color, const ViewDesc* views,
+bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                     int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                     cudaStream_t stream, unsigned long long* counts = nullptr,
                     uint8_t* block_bits = nullptr, const int* tile_order = nullptr,
@@ -138,8 +136,7 @@ bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const float2
 // The adjoint. `block_bits`, when the forward wrote them, replace the
 // geometric warp masks in the two-pixel form: a warp walks only the entries
 // one of its pixels took.
-void launch_backward(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                     const float4* conic_op, const float4* color, const ViewDesc* views,
+void launch_backward(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                      int n_views, int total_tiles, const float* T_final, const int32_t* last,
                      const float* dL_drgb, ScreenGrad* screen, cudaStream_t stream,
                      const uint8_t* block_bits = nullptr, const int* tile_order = nullptr,

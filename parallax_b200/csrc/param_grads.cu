@@ -310,7 +310,7 @@ template <int S>
 __global__ void __launch_bounds__(kParamThreads, 3)
     k_param_grads(const float* __restrict__ params, int N, int64_t slot_stride,
                   const ViewDesc* __restrict__ views, int n_views, const uint32_t* depth_key,
-                  const float4* __restrict__ conic_op, const float4* __restrict__ color,
+                  const SlotGeom* __restrict__ geom, const float4* __restrict__ color,
                   const ScreenGrad* __restrict__ screen, float* __restrict__ grads,
                   float* __restrict__ screen_gradient, int32_t* __restrict__ visible_count) {
   constexpr int T = kParamThreads;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kParamThreads, 3)
         const int go = blockIdx.x * T + owner;
         const int64_t slot = v * slot_stride + (go - vd.gauss_offset);
         const ScreenGrad sg = screen[slot];
-        const float4 co = conic_op[slot];
+        const float4 co = geom[slot].conic_op;
         const float4 col = color[slot];
         const float pos[3] = {s_state[0][owner], s_state[1][owner], s_state[2][owner]};
         const float qn[4] = {s_state[3][owner], s_state[4][owner], s_state[5][owner],
@@ -490,7 +490,7 @@ void configure_param_grads_kernel() {
 
 void launch_param_grads(const float* params, int N, int S, int64_t slot_stride,
                         const ViewDesc* views, int n_views, const uint32_t* depth_key,
-                        const float4* conic_op, const float4* color, const ScreenGrad* screen,
+                        const SlotGeom* geom, const float4* color, const ScreenGrad* screen,
                         float* grads, float* screen_gradient, int32_t* visible_count,
                         cudaStream_t stream) {
   const int threads = kParamThreads;
@@ -499,7 +499,7 @@ void launch_param_grads(const float* params, int N, int S, int64_t slot_stride,
 #define LAUNCH(SS)                                                                      \
   count_launch();                                                                       \
   k_param_grads<SS><<<blocks, threads, sizeof(ParamSmem<SS>), stream>>>(                \
-      params, N, slot_stride, views, n_views, depth_key, conic_op, color, screen, grads, \
+      params, N, slot_stride, views, n_views, depth_key, geom, color, screen, grads, \
       screen_gradient, visible_count)
   switch (S) {
     case 0: LAUNCH(0); break;

@@ -137,8 +137,9 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
       }
     }
     const float conic_a = cov[3] / det, conic_b = -cov[1] / det, conic_c = cov[0] / det;
-    out.xy[slot] = make_float2(mean_x, mean_y);
-    out.conic_op[slot] = make_float4(conic_a, conic_b, conic_c, st.opacity);
+    SlotGeom geom;
+    geom.xy = make_float2(mean_x, mean_y);
+    geom.conic_op = make_float4(conic_a, conic_b, conic_c, st.opacity);
     out.color[slot] = make_float4(color[0], color[1], color[2], __uint_as_float(flags));
     out.depth_key[slot] = __float_as_uint(p[2]);
     if (out.debug_cov != nullptr)
@@ -152,8 +153,7 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
     int y0 = max(0, float_to_int_x86(floorf((mean_y - radius) / 16.f)));
     int y1 = min(vd.tiles_y - 1, float_to_int_x86(floorf((mean_y + radius) / 16.f)));
     if (tight) {
-      const Footprint f =
-          splat_footprint(make_float4(conic_a, conic_b, conic_c, st.opacity), vd.min_alpha);
+      const Footprint f = splat_footprint(geom.conic_op, vd.min_alpha);
       if (!f.all) {
         x0 = max(x0, first_tile(mean_x - f.ex));
         x1 = min(x1, last_tile(mean_x + f.ex));
@@ -165,8 +165,9 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
         }
       }
     }
-    out.rect[slot] = make_uint2((uint32_t)(x0 & 0xFFFF) | ((uint32_t)(x1 & 0xFFFF) << 16),
-                                (uint32_t)(y0 & 0xFFFF) | ((uint32_t)(y1 & 0xFFFF) << 16));
+    geom.rect = make_uint2((uint32_t)(x0 & 0xFFFF) | ((uint32_t)(x1 & 0xFFFF) << 16),
+                           (uint32_t)(y0 & 0xFFFF) | ((uint32_t)(y1 & 0xFFFF) << 16));
+    out.geom[slot] = geom;
   }
 }
 

@@ -31,7 +31,7 @@ RasterConfig& raster_config() {
 template <bool kCount, int PX>
 __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
     k_forward(const int2* __restrict__ ranges, const uint32_t* __restrict__ pair_slots,
-              const float2* __restrict__ xy, const float4* __restrict__ conic_op,
+              const SlotGeom* __restrict__ geom,
               const float4* __restrict__ color, const ViewDesc* __restrict__ views, int n_views,
               float* __restrict__ rgb_out, float* __restrict__ T_out,
               int32_t* __restrict__ last_out, unsigned long long* __restrict__ counts) {
@@ -64,8 +64,8 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
     const int n = min(kBatch, info.range.y - base);
     for (int i = threadIdx.x; i < n; i += kThreads) {
       const uint32_t slot = pair_slots[base + i];
-      const float4 co = conic_op[slot];
-      const float2 mean = xy[slot];
+      const float4 co = geom[slot].conic_op;
+      const float2 mean = geom[slot].xy;
       float4 c = color[slot];
       c.w = power_floor(co.w, min_alpha);
       s_xy[i] = mean;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
 template <bool kCount, bool kBits, int kFwdBatch>
 __global__ void __launch_bounds__(TileGeom<2>::kThreads, 8)
     k_forward_x2(const int2* __restrict__ ranges, const uint32_t* __restrict__ pair_slots,
-                 const float2* __restrict__ xy, const float4* __restrict__ conic_op,
+                 const SlotGeom* __restrict__ geom,
                  const float4* __restrict__ color, const ViewDesc* __restrict__ views,
                  int n_views, float* __restrict__ rgb_out, float* __restrict__ T_out,
                  int32_t* __restrict__ last_out, unsigned long long* __restrict__ counts,
@@ -207,8 +207,8 @@ __global__ void __launch_bounds__(TileGeom<2>::kThreads, 8)
         for (int w = 0; w < TileGeom<2>::kWarps; ++w) s_took[w][i] = 0;
       }
       const uint32_t slot = pair_slots[base + i];
-      const float4 co = conic_op[slot];
-      const float2 mean = xy[slot];
+      const float4 co = geom[slot].conic_op;
+      const float2 mean = geom[slot].xy;
       const float4 c = color[slot];
       // staged negated (see visit): the mean, the opacity and the colour
       s_xy[i] = make_float2(-mean.x, -mean.y);
@@ -382,19 +382,17 @@ void launch_tile_order(const int2* ranges, int total_tiles, int* order, int* wor
 namespace {
 
 template <bool kCount, int PX>
-void forward_px(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                const float4* conic_op, const float4* color, const ViewDesc* views, int n_views,
+void forward_px(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views, int n_views,
                 int total_tiles, float* rgb, float* T, int32_t* last, cudaStream_t stream,
                 unsigned long long* counts) {
   k_forward<kCount, PX><<<total_tiles, TileGeom<PX>::kThreads, 0, stream>>>(
-      ranges, pair_slots, xy, conic_op, color, views, n_views, rgb, T, last, counts);
+      ranges, pair_slots, geom, color, views, n_views, rgb, T, last, counts);
 }
 
 // The two-pixel kernel at the configured batch and schedule. The counting
 // form always runs one CTA per tile in tile order.
 template <bool kCount, bool kBits, int B>
-void forward_x2_launch(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                       const float4* conic_op, const float4* color, const ViewDesc* views,
+void forward_x2_launch(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                        int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                        cudaStream_t stream, unsigned long long* counts, uint8_t* bits,
                        const int* order, int* ticket) {
@@ -407,18 +405,17 @@ void forward_x2_launch(const int2* ranges, const uint32_t* pair_slots, const flo
     cudaMemsetAsync(ticket, 0, sizeof(int), stream);
   }
   k_forward_x2<kCount, kBits, B><<<grid, TileGeom<2>::kThreads, 0, stream>>>(
-      ranges, pair_slots, xy, conic_op, color, views, n_views, rgb, T, last, counts, bits,
+      ranges, pair_slots, geom, color, views, n_views, rgb, T, last, counts, bits,
       schedule, order, ticket, total_tiles);
 }
 
 template <bool kCount>
-void forward_x2_dispatch(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                         const float4* conic_op, const float4* color, const ViewDesc* views,
+void forward_x2_dispatch(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                          int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                          cudaStream_t stream, unsigned long long* counts, uint8_t* bits,
                          const int* order, int* ticket) {
 #define PXS_FWD(BITS, B)                                                                    \
-  forward_x2_launch<kCount, BITS, B>(ranges, pair_slots, xy, conic_op, color, views, n_views, \
+  forward_x2_launch<kCount, BITS, B>(ranges, pair_slots, geom, color, views, n_views, \
                                      total_tiles, rgb, T, last, stream, counts, bits, order,  \
                                      ticket)
   const int b = raster_config().forward_batch;
@@ -435,22 +432,21 @@ void forward_x2_dispatch(const int2* ranges, const uint32_t* pair_slots, const f
 }
 
 template <bool kCount>
-void forward_dispatch(int px, const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                      const float4* conic_op, const float4* color, const ViewDesc* views,
+void forward_dispatch(int px, const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                       int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                       cudaStream_t stream, unsigned long long* counts, uint8_t* bits,
                       const int* order, int* ticket) {
   switch (px) {
     case 1:
-      forward_px<kCount, 1>(ranges, pair_slots, xy, conic_op, color, views, n_views,
+      forward_px<kCount, 1>(ranges, pair_slots, geom, color, views, n_views,
                             total_tiles, rgb, T, last, stream, counts);
       break;
     case 4:
-      forward_px<kCount, 4>(ranges, pair_slots, xy, conic_op, color, views, n_views,
+      forward_px<kCount, 4>(ranges, pair_slots, geom, color, views, n_views,
                             total_tiles, rgb, T, last, stream, counts);
       break;
     default:
-      forward_x2_dispatch<kCount>(ranges, pair_slots, xy, conic_op, color, views, n_views,
+      forward_x2_dispatch<kCount>(ranges, pair_slots, geom, color, views, n_views,
                                   total_tiles, rgb, T, last, stream, counts, bits, order,
                                   ticket);
   }
@@ -458,8 +454,7 @@ void forward_dispatch(int px, const int2* ranges, const uint32_t* pair_slots, co
 
 }  // namespace
 
-bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                    const float4* conic_op, const float4* color, const ViewDesc* views,
+bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                     int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                     cudaStream_t stream, unsigned long long* counts, uint8_t* block_bits,
                     const int* tile_order, int* ticket) {
@@ -468,10 +463,10 @@ bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const float2
   const int px = raster_config().forward_px;
   uint8_t* bits = (px == 1 || px == 4) ? nullptr : block_bits;
   if (counts != nullptr)
-    forward_dispatch<true>(px, ranges, pair_slots, xy, conic_op, color, views, n_views,
+    forward_dispatch<true>(px, ranges, pair_slots, geom, color, views, n_views,
                            total_tiles, rgb, T, last, stream, counts, bits, tile_order, ticket);
   else
-    forward_dispatch<false>(px, ranges, pair_slots, xy, conic_op, color, views, n_views,
+    forward_dispatch<false>(px, ranges, pair_slots, geom, color, views, n_views,
                             total_tiles, rgb, T, last, stream, nullptr, bits, tile_order,
                             ticket);
   return bits != nullptr;

@@ -95,7 +95,7 @@ __device__ __forceinline__ void add_entry(ScreenGrad* slot, const LaneSums& v, b
 template <int PX>
 __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
     k_backward(const int2* __restrict__ ranges, const uint32_t* __restrict__ pair_slots,
-               const float2* __restrict__ xy, const float4* __restrict__ conic_op,
+               const SlotGeom* __restrict__ geom,
                const float4* __restrict__ color, const ViewDesc* __restrict__ views,
                int n_views, const float* __restrict__ T_final,
                const int32_t* __restrict__ last_in, const float* __restrict__ dL_drgb,
@@ -151,8 +151,8 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += kThreads) {
       const uint32_t slot = pair_slots[batch_start + i];
-      const float4 co = conic_op[slot];
-      const float2 mean = xy[slot];
+      const float4 co = geom[slot].conic_op;
+      const float2 mean = geom[slot].xy;
       float4 c = color[slot];
       c.w = power_floor(co.w, min_alpha);
       s_slot[i] = slot;
@@ -256,7 +256,7 @@ __device__ __forceinline__ uint32_t mask_from_block_bits(uint32_t bits) {
 template <int NP, int kB, bool kBits>
 __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
     k_backward_pairs(const int2* __restrict__ ranges, const uint32_t* __restrict__ pair_slots,
-                     const float2* __restrict__ xy, const float4* __restrict__ conic_op,
+                     const SlotGeom* __restrict__ geom,
                      const float4* __restrict__ color, const ViewDesc* __restrict__ views,
                      int n_views, const float* __restrict__ T_final,
                      const int32_t* __restrict__ last_in, const float* __restrict__ dL_drgb,
@@ -328,8 +328,8 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
     __syncthreads();
     for (int i = threadIdx.x; i < n; i += kThreads) {
       const uint32_t slot = pair_slots[batch_start + i];
-      const float4 co = conic_op[slot];
-      const float2 mean = xy[slot];
+      const float4 co = geom[slot].conic_op;
+      const float2 mean = geom[slot].xy;
       s_slot[i] = slot;
       s_xy[i] = make_float2(-mean.x, -mean.y);  // negated: fx + (-mx) is fx - mx
       s_co[i] = make_float4(co.x, co.y, co.z, -co.w);
@@ -455,19 +455,17 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
 namespace {
 
 template <int PX>
-void backward_px(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                 const float4* conic_op, const float4* color, const ViewDesc* views, int n_views,
+void backward_px(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views, int n_views,
                  int total_tiles, const float* T_final, const int32_t* last,
                  const float* dL_drgb, ScreenGrad* screen, cudaStream_t stream) {
   k_backward<PX><<<total_tiles, TileGeom<PX>::kThreads, 0, stream>>>(
-      ranges, pair_slots, xy, conic_op, color, views, n_views, T_final, last, dL_drgb, screen);
+      ranges, pair_slots, geom, color, views, n_views, T_final, last, dL_drgb, screen);
 }
 
 }  // namespace
 
 template <int NP, int B, bool kBits>
-void backward_pairs_launch(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                           const float4* conic_op, const float4* color, const ViewDesc* views,
+void backward_pairs_launch(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                            int n_views, int total_tiles, const float* T_final,
                            const int32_t* last, const float* dL_drgb, ScreenGrad* screen,
                            cudaStream_t stream, const uint8_t* block_bits,
@@ -480,12 +478,11 @@ void backward_pairs_launch(const int2* ranges, const uint32_t* pair_slots, const
     cudaMemsetAsync(ticket, 0, sizeof(int), stream);
   }
   k_backward_pairs<NP, B, kBits><<<grid, TileGeom<2 * NP>::kThreads, 0, stream>>>(
-      ranges, pair_slots, xy, conic_op, color, views, n_views, T_final, last, dL_drgb, screen,
+      ranges, pair_slots, geom, color, views, n_views, T_final, last, dL_drgb, screen,
       block_bits, schedule, tile_order, ticket, total_tiles);
 }
 
-void launch_backward(const int2* ranges, const uint32_t* pair_slots, const float2* xy,
-                     const float4* conic_op, const float4* color, const ViewDesc* views,
+void launch_backward(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                      int n_views, int total_tiles, const float* T_final, const int32_t* last,
                      const float* dL_drgb, ScreenGrad* screen, cudaStream_t stream,
                      const uint8_t* block_bits, const int* tile_order, int* ticket) {
@@ -493,15 +490,15 @@ void launch_backward(const int2* ranges, const uint32_t* pair_slots, const float
   count_launch();
 #define PXS_BWD(NP, B)                                                                         \
   (block_bits != nullptr                                                                       \
-       ? backward_pairs_launch<NP, B, true>(ranges, pair_slots, xy, conic_op, color, views,    \
+       ? backward_pairs_launch<NP, B, true>(ranges, pair_slots, geom, color, views,    \
                                             n_views, total_tiles, T_final, last, dL_drgb,      \
                                             screen, stream, block_bits, tile_order, ticket)    \
-       : backward_pairs_launch<NP, B, false>(ranges, pair_slots, xy, conic_op, color, views,   \
+       : backward_pairs_launch<NP, B, false>(ranges, pair_slots, geom, color, views,   \
                                              n_views, total_tiles, T_final, last, dL_drgb,     \
                                              screen, stream, block_bits, tile_order, ticket))
   switch (raster_config().backward_px) {
     case 1:
-      backward_px<1>(ranges, pair_slots, xy, conic_op, color, views, n_views, total_tiles,
+      backward_px<1>(ranges, pair_slots, geom, color, views, n_views, total_tiles,
                      T_final, last, dL_drgb, screen, stream);
       break;
     case 4:

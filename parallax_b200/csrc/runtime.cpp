@@ -124,11 +124,9 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   if (V > 0)
     PXS_CUDA(cudaMemcpyAsync(d_views.get(), batch.views.data(), sizeof(ViewDesc) * V,
                              cudaMemcpyHostToDevice, stream));
-  xy.reserve(slots);
-  conic_op.reserve(slots);
+  geom.reserve(slots);
   color.reserve(slots);
   depth_key.reserve(slots);
-  rect.reserve(slots);
   sort_keys.reserve(slots);
   sort_vals.reserve(slots);
   sort_keys_alt.reserve(slots);
@@ -206,11 +204,9 @@ void Frame::project(const float* params, cudaStream_t stream, bool want_debug,
                     bool whole_lists) {
   whole_lists_ = whole_lists;
   ProjectedSoA out;
-  out.xy = xy.get();
-  out.conic_op = conic_op.get();
+  out.geom = geom.get();
   out.color = color.get();
   out.depth_key = depth_key.get();
-  out.rect = rect.get();
   out.debug_cov = nullptr;
   if (want_debug) out.debug_cov = debug_cov.reserve(static_cast<size_t>(V) * slot_stride);
   launch_project(params, N, S, slot_stride, d_views.get(), V, out, !whole_lists, stream);
@@ -238,7 +234,7 @@ int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
   //    order, then each chunk writes its records at its bases
   const int cpv = slot_chunks_per_view(slot_stride);
   const int64_t n_row_chunks = static_cast<int64_t>(batch.total_rows) * cpv;
-  launch_slot_row_counts(v, k, rect.get(), d_views.get(), V, slot_stride,
+  launch_slot_row_counts(v, k, geom.get(), d_views.get(), V, slot_stride,
                          batch.max_tiles_y, row_chunk_counts.get(), stream);
   exclusive_scan_i32_to_i64(row_chunk_counts.get(), row_chunk_offsets.get(), n_row_chunks,
                             d_total_records.get(), scan_, stream);
@@ -253,8 +249,7 @@ int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
     throw Error(PXS_ERR_INVALID, "pair buffers must be reserved before an unsynchronised bin");
   }
   PXS_CUDA(cudaMemsetAsync(overflow.get(), 0, sizeof(int32_t), stream));
-  launch_slot_row_expand(v, k, rect.get(), whole_lists_ ? nullptr : xy.get(),
-                         whole_lists_ ? nullptr : conic_op.get(), d_views.get(), V, slot_stride,
+  launch_slot_row_expand(v, k, geom.get(), !whole_lists_, d_views.get(), V, slot_stride,
                          batch.max_tiles_y, row_chunk_offsets.get(), record_capacity,
                          rec_vals.get(), rec_xr.get(), stream);
   launch_row_ranges_from_chunks(row_chunk_offsets.get(), batch.total_rows, cpv,
@@ -302,7 +297,7 @@ const int* Frame::ordered_tiles(int schedule, cudaStream_t stream) {
 void Frame::forward(cudaStream_t stream, unsigned long long* counts) {
   const int* order = counts ? nullptr : ordered_tiles(raster_config().forward_schedule, stream);
   have_block_bits =
-      launch_forward(ranges.get(), sorted_pair_vals, xy.get(), conic_op.get(), color.get(),
+      launch_forward(ranges.get(), sorted_pair_vals, geom.get(), color.get(),
                      d_views.get(), V, batch.total_tiles, rgb.get(), transmittance.get(),
                      last.get(), stream, counts, block_bits.get(), order, tickets.get());
   PXS_CUDA(cudaGetLastError());
@@ -325,7 +320,7 @@ void Frame::backward(const float* dL_drgb, cudaStream_t stream) {
   const size_t slots = static_cast<size_t>(V) * static_cast<size_t>(slot_stride);
   PXS_CUDA(cudaMemsetAsync(screen.get(), 0, sizeof(ScreenGrad) * slots, stream));
   const int* order = ordered_tiles(raster_config().backward_schedule, stream);
-  launch_backward(ranges.get(), sorted_pair_vals, xy.get(), conic_op.get(), color.get(),
+  launch_backward(ranges.get(), sorted_pair_vals, geom.get(), color.get(),
                   d_views.get(), V, batch.total_tiles, transmittance.get(), last.get(), dL_drgb,
                   screen.get(), stream, have_block_bits ? block_bits.get() : nullptr, order,
                   tickets.get() + 1);
@@ -334,7 +329,7 @@ void Frame::backward(const float* dL_drgb, cudaStream_t stream) {
 
 void Frame::param_grads(const float* params, float* grads, float* screen_gradient,
                         int32_t* visible_count, cudaStream_t stream) {
-  launch_param_grads(params, N, S, slot_stride, d_views.get(), V, depth_key.get(), conic_op.get(),
+  launch_param_grads(params, N, S, slot_stride, d_views.get(), V, depth_key.get(), geom.get(),
                      color.get(), screen.get(), grads, screen_gradient, visible_count, stream);
   PXS_CUDA(cudaGetLastError());
 }

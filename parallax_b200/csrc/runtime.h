@@ -152,10 +152,9 @@ class Frame {
 
   // device buffers
   DeviceArray<ViewDesc> d_views;
-  DeviceArray<float2> xy;
-  DeviceArray<float4> conic_op, color, debug_cov;
+  DeviceArray<SlotGeom> geom;
+  DeviceArray<float4> color, debug_cov;
   DeviceArray<uint32_t> depth_key;
-  DeviceArray<uint2> rect;
   DeviceArray<uint32_t> sort_keys, sort_vals, sort_keys_alt, sort_vals_alt;
   // per (tile row, chunk of depth-sorted slots): records and their offsets
   DeviceArray<int32_t> row_chunk_counts;

@@ -38,7 +38,8 @@ struct ViewDesc {
   float min_alpha;
   float transmittance_cutoff;
   float screen_dilation;
-  int32_t loss_tile_offset;  // first output tile of this view in the loss kernel's flat grid
+  int32_t loss_tile_offset;  // first CTA of this view in the loss kernel's grid
+  int32_t l1_block_offset;   // the same for the loss without SSIM
   int64_t target_offset;     // first pixel of this view's target image
   // the gaussians this view renders: [gauss_offset, gauss_offset + gauss_count)
   // of the parameter arrays; slot v * slot_stride + i holds gaussian

@@ -143,17 +143,17 @@ void launch_backward(const int2* ranges, const uint32_t* pair_slots, const SlotG
                      int* ticket = nullptr);
 
 // loss.cu
-size_t loss_smem_bytes();
-void configure_loss_kernel();  // once per device, outside graph capture
-// Output tiles of one view in the loss kernel.
-int64_t loss_tiles(int width, int height);
-// `flat_tiles` >= 0: a one-dimensional grid of that many CTAs over every
-// view's own tiles (the sum of loss_tiles over the views); otherwise a grid
-// sized for the largest view.
+// CTAs of the loss over one image: `rows` output rows each (loss_rows), or with
+// rows = 0 the elementwise loss without SSIM.
+int64_t loss_blocks(int width, int height, int rows);
+// Output rows per CTA for these images together.
+int loss_rows(const int* widths, const int* heights, int n);
+// One launch over every view's own CTAs, `blocks` in all, found by the views'
+// loss_tile_offset (rows > 0) or l1_block_offset (rows = 0). `sums`: 2 n_views + 1
+// doubles.
 void launch_loss(const float* rendered, const float* target, const ViewDesc* views, int n_views,
-                 int max_width, int max_height, const LossParams& lp, float* grad_out,
-                 double* sums, float* per_view, float* total, cudaStream_t stream,
-                 int64_t flat_tiles = -1);
+                 int64_t blocks, int rows, const LossParams& lp, float* grad_out, double* sums,
+                 float* per_view, float* total, cudaStream_t stream);
 
 // export.cu: the reference's file formats packed on the device
 void launch_pack_ply(const float* params, int n, const int* field_src, int fields, float* out,

@@ -50,7 +50,6 @@ ViewBatch make_batch(const pxs_camera* cameras, int n_views, const pxs_raster_op
   ViewBatch b;
   b.views.resize(static_cast<size_t>(n_views));
   int tile_offset = 0, row_offset = 0;
-  int64_t loss_tile_offset = 0;
   int64_t pixel_offset = 0;
   for (int v = 0; v < n_views; ++v) {
     ViewDesc& d = b.views[static_cast<size_t>(v)];
@@ -65,8 +64,6 @@ ViewBatch make_batch(const pxs_camera* cameras, int n_views, const pxs_raster_op
       throw Error(PXS_ERR_INVALID, "image too large (at most 2048 tiles across and down)");
     d.tile_offset = tile_offset;
     d.row_offset = row_offset;
-    d.loss_tile_offset = static_cast<int32_t>(loss_tile_offset);
-    loss_tile_offset += loss_tiles(d.cam.width, d.cam.height);
     d.pixel_offset = pixel_offset;
     d.target_offset = pixel_offset;
     d.min_alpha = options.min_alpha;
@@ -77,8 +74,18 @@ ViewBatch make_batch(const pxs_camera* cameras, int n_views, const pxs_raster_op
     b.max_tiles_x = std::max(b.max_tiles_x, d.tiles_x);
     b.max_tiles_y = std::max(b.max_tiles_y, d.tiles_y);
     pixel_offset += static_cast<int64_t>(d.cam.width) * d.cam.height;
-    b.max_width = std::max(b.max_width, d.cam.width);
-    b.max_height = std::max(b.max_height, d.cam.height);
+  }
+  std::vector<int> widths, heights;
+  for (const ViewDesc& d : b.views) {
+    widths.push_back(d.cam.width);
+    heights.push_back(d.cam.height);
+  }
+  b.loss_rows = loss_rows(widths.data(), heights.data(), n_views);
+  for (ViewDesc& d : b.views) {
+    d.loss_tile_offset = static_cast<int32_t>(b.loss_blocks);
+    d.l1_block_offset = static_cast<int32_t>(b.l1_blocks);
+    b.loss_blocks += loss_blocks(d.cam.width, d.cam.height, b.loss_rows);
+    b.l1_blocks += loss_blocks(d.cam.width, d.cam.height, 0);
   }
   b.total_pixels = pixel_offset;
   b.total_tiles = tile_offset;
@@ -97,7 +104,6 @@ void Frame::ensure_scan_scratch(int64_t n) {
 
 void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   if (!configured_) {
-    configure_loss_kernel();
     configure_bin_kernels();
     configure_param_grads_kernel();
     PXS_CUDA(cudaGetLastError());
@@ -153,7 +159,7 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   row_ranges.reserve(static_cast<size_t>(std::max(batch.total_rows, 1)));
   n_chunks.reserve(1);
   d_total_records.reserve(1);
-  loss_sums.reserve(static_cast<size_t>(2 * std::max(V, 1)));
+  loss_sums.reserve(static_cast<size_t>(2 * std::max(V, 1) + 1));
   loss_per_view.reserve(static_cast<size_t>(std::max(V, 1)));
   loss_total.reserve(1);
   // the depth sort's histograms; the tile sort's are sized in reserve_pairs
@@ -309,10 +315,10 @@ void Frame::loss(const float* target, float ssim_weight, int mode, float* grad_o
   ssim_kernel_weights(lp.kernel);
   lp.ssim_weight = ssim_weight;
   lp.mode = mode;
-  int64_t tiles = 0;
-  for (const ViewDesc& d : batch.views) tiles += loss_tiles(d.cam.width, d.cam.height);
-  launch_loss(rgb.get(), target, d_views.get(), V, batch.max_width, batch.max_height, lp,
-              grad_out, loss_sums.get(), loss_per_view.get(), loss_total.get(), stream, tiles);
+  const bool ssim = mode == 1 || ssim_weight > 0.f;
+  launch_loss(rgb.get(), target, d_views.get(), V, ssim ? batch.loss_blocks : batch.l1_blocks,
+              ssim ? batch.loss_rows : 0, lp, grad_out, loss_sums.get(), loss_per_view.get(),
+              loss_total.get(), stream);
   PXS_CUDA(cudaGetLastError());
 }
 

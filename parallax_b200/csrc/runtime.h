@@ -93,7 +93,8 @@ struct ViewBatch {
   int total_tiles = 0;
   int total_rows = 0;       // tile rows over all views
   int max_tiles_x = 0, max_tiles_y = 0;
-  int max_width = 0, max_height = 0;
+  int loss_rows = 0;        // output rows per CTA of the loss
+  int64_t loss_blocks = 0, l1_blocks = 0;
   // the views carry their own gaussian ranges (several scenes); otherwise
   // Frame::prepare gives every view the whole cloud
   bool own_ranges = false;

@@ -268,11 +268,12 @@ __global__ void k_finish_keys(const float* __restrict__ params, int N,
 }
 
 __global__ void k_gather_params(const float* __restrict__ params, int N, int P,
-                                const uint32_t* __restrict__ order, int64_t n_new,
+                                const uint32_t* __restrict__ order,
+                                const uint32_t* __restrict__ source, int64_t n_new,
                                 float* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_new) return;
-  const int64_t g = order[i];
+  const int64_t g = source[order[i]];
   for (int c = 0; c < P; ++c) out[(int64_t)c * n_new + i] = params[(int64_t)c * N + g];
 }
 
@@ -407,12 +408,12 @@ int64_t finish_device(DensifyWork& w, const float* params, int N, int S, float m
   int32_t* keep = w.keep.reserve(n);
   int64_t* keep_off = w.keep_offset.reserve(n);
   int64_t* totals = w.totals.reserve(4);
-  const size_t scratch =
-      std::max(scan_scratch_bytes(static_cast<int64_t>(n)),
-               scan_scratch_bytes(static_cast<int64_t>(radix_hist_entries(N, 0, 9))));
-  char* base = w.scan.reserve(scratch + 64);
+  // the sort takes whole tiles: the last one is filled with the greatest key
+  const int64_t padded = round_up(N, kSortTile);
+  const int64_t widest = std::max<int64_t>(N, depth_sort_hist_entries(padded, padded));
+  char* base = w.scan.reserve(scan_scratch_bytes(widest) + 64);
   ScanScratch ss;
-  scan_scratch_assign(ss, base, std::max<int64_t>(N, radix_hist_entries(N, 0, 9)));
+  scan_scratch_assign(ss, base, widest);
   const unsigned blocks = (N + 255) / 256;
   count_launch();
   k_finish_keep<<<blocks, 256, 0, stream>>>(params, N, min_opacity, 1e3f, keep);
@@ -421,19 +422,22 @@ int64_t finish_device(DensifyWork& w, const float* params, int N, int S, float m
   PXS_CUDA(cudaMemcpyAsync(&kept, totals, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
   PXS_CUDA(cudaStreamSynchronize(stream));
   if (kept == 0) return 0;
-  uint32_t* keys = w.sort_a.reserve(n);
-  uint32_t* vals = w.sort_b.reserve(n);
-  uint32_t* keys_alt = w.sort_c.reserve(n);
-  uint32_t* vals_alt = w.sort_d.reserve(n);
-  const size_t hist_n = radix_hist_entries(kept, 0, 9);
+  const int64_t sorted = round_up(kept, kSortTile);
+  uint32_t* keys = w.sort_a.reserve(static_cast<size_t>(padded));
+  uint32_t* source = w.sort_b.reserve(n);
+  uint32_t* buffers[4];
+  for (int i = 0; i < 4; ++i) buffers[i] = w.sorted[i].reserve(static_cast<size_t>(padded));
+  const size_t hist_n = depth_sort_hist_entries(sorted, sorted);
   uint32_t* hist = w.hist.reserve(hist_n);
   uint32_t* hist_scanned = w.hist_scanned.reserve(hist_n);
   count_launch();
-  k_finish_keys<<<blocks, 256, 0, stream>>>(params, N, keep, keep_off, keys, vals);
-  radix_sort_pairs(keys, vals, keys_alt, vals_alt, kept, 0, 32, hist, hist_scanned, ss, stream);
+  k_finish_keys<<<blocks, 256, 0, stream>>>(params, N, keep, keep_off, keys, source);
+  PXS_CUDA(cudaMemsetAsync(keys + kept, 0xFF, sizeof(uint32_t) * (sorted - kept), stream));
+  depth_sort(keys, sorted, sorted, buffers[0], buffers[1], buffers[2], buffers[3], hist,
+             hist_scanned, ss, stream);
   count_launch();
-  k_gather_params<<<(unsigned)((kept + 255) / 256), 256, 0, stream>>>(params, N, P, vals, kept,
-                                                                      out);
+  k_gather_params<<<(unsigned)((kept + 255) / 256), 256, 0, stream>>>(params, N, P, buffers[3],
+                                                                      source, kept, out);
   PXS_CUDA(cudaGetLastError());
   return kept;
 }

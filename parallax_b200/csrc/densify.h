@@ -34,7 +34,7 @@ struct DensifyWork {
   DeviceArray<int64_t> keep_offset, add_offset, split_rank, np_rank, totals;
   DeviceArray<float> adds;
   DeviceArray<char> scan;
-  DeviceArray<uint32_t> jump_cols, sort_a, sort_b, sort_c, sort_d, hist, hist_scanned;
+  DeviceArray<uint32_t> jump_cols, sort_a, sort_b, sorted[4], hist, hist_scanned;
   uint32_t host_cols[32 * kJumpPowers];
 };
 

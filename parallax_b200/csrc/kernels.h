@@ -48,16 +48,14 @@ void exclusive_scan_i32_to_i64(const int32_t* in, int64_t* out, int64_t n, int64
                                ScanScratch& scratch, cudaStream_t stream);
 void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, ScanScratch& scratch,
                         cudaStream_t stream);
-size_t radix_hist_entries(int64_t n, int64_t segment_len, int max_bits);
-// Sorts (keys, vals) by the low `total_bits` bits of the keys, stably, each
-// `segment_len` run independently (segment_len a multiple of kSortTile, or 0
-// for one segment). keys/vals and the *_alt buffers are swapped so that on
-// return keys/vals hold the result. Returns the number of passes.
-int radix_sort_pairs(uint32_t*& keys, uint32_t*& vals, uint32_t*& keys_alt,
-                     uint32_t*& vals_alt, int64_t n, int64_t segment_len, int total_bits,
-                     uint32_t* hist, uint32_t* hist_scanned, ScanScratch& scratch,
-                     cudaStream_t stream, const int64_t* n_device = nullptr);
-void launch_iota(uint32_t* out, int64_t n, cudaStream_t stream);
+// Sorts n keys with their places as values, stably, each `segment_len` run
+// independently (both multiples of kSortTile), into keys_b and vals_b; the a
+// buffers are scratch, as are hist (depth_sort_hist_entries) and hist_scanned (as
+// large).
+size_t depth_sort_hist_entries(int64_t n, int64_t segment_len);
+void depth_sort(const uint32_t* keys, int64_t n, int64_t segment_len, uint32_t* keys_a,
+                uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, uint32_t* hist,
+                uint32_t* hist_scanned, ScanScratch& scratch, cudaStream_t stream);
 
 // bin.cu
 void configure_bin_kernels();  // once per device, outside graph capture

@@ -162,8 +162,7 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   loss_sums.reserve(static_cast<size_t>(2 * std::max(V, 1) + 1));
   loss_per_view.reserve(static_cast<size_t>(std::max(V, 1)));
   loss_total.reserve(1);
-  // the depth sort's histograms; the tile sort's are sized in reserve_pairs
-  const size_t depth_hist = radix_hist_entries(static_cast<int64_t>(slots), slot_stride, 8);
+  const size_t depth_hist = depth_sort_hist_entries(static_cast<int64_t>(slots), slot_stride);
   if (hist.capacity() < depth_hist) {
     hist.reserve(depth_hist);
     hist_scanned.reserve(depth_hist);
@@ -227,14 +226,11 @@ int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
     return 0;
   }
   // 1. every slot near to far within its view (stable: equal depths by index)
-  PXS_CUDA(cudaMemcpyAsync(sort_keys.get(), depth_key.get(), sizeof(uint32_t) * slots,
-                           cudaMemcpyDeviceToDevice, stream));
-  launch_iota(sort_vals.get(), slots, stream);
-  uint32_t *k = sort_keys.get(), *v = sort_vals.get();
-  uint32_t *ka = sort_keys_alt.get(), *va = sort_vals_alt.get();
-  radix_sort_pairs(k, v, ka, va, slots, slot_stride, 32, hist.get(), hist_scanned.get(), scan_,
-                   stream);
-  sorted_slots = v;  // k holds their keys: kCulledKey for a culled slot
+  depth_sort(depth_key.get(), slots, slot_stride, sort_keys_alt.get(), sort_vals_alt.get(),
+             sort_keys.get(), sort_vals.get(), hist.get(), hist_scanned.get(), scan_, stream);
+  const uint32_t* const k = sort_keys.get();  // kCulledKey for a culled slot
+  uint32_t* const v = sort_vals.get();
+  sorted_slots = v;
   // 2. one record per covered tile row, grouped by row and near to far within
   //    a row: per (view, slot chunk) row counts, their scan in (row, chunk)
   //    order, then each chunk writes its records at its bases

@@ -1,9 +1,9 @@
-// sort.cu -- scans, radix sort and key ranges for the binning path.
+// sort.cu -- scans and the depth sort for the binning path.
 //
-// Device-wide exclusive scans, a stable segmented LSD radix sort of 32-bit
-// keys with 32-bit values, and the range kernel. The binning path uses them
-// for the depth sort of every (view, gaussian) slot (segmented per view; ties
-// keep gaussian order) and for grouping the tile-row records by row (bin.cu).
+// Device-wide exclusive scans, and a stable segmented LSD radix sort of the depth
+// keys of every (view, gaussian) slot with the slots as values (segmented per
+// view; ties keep gaussian order), four passes of 8 bits. The first pass reads
+// the keys where projection left them and counts the slots itself.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -13,7 +13,6 @@ namespace {
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
-constexpr int kMaxBins = 512;
 constexpr int kSortWarps = kSortThreads / 32;
 
 template <typename T>
@@ -90,166 +89,159 @@ __global__ void __launch_bounds__(kScanThreads)
 
 // ------------------------------------------------------------ radix sort
 
-struct RadixPass {
-  int shift;
-  int bits;
-  int64_t n;                // items (an upper bound when n_device is set)
-  const int64_t* n_device;  // optional device-side item count
-  int64_t segment_len;      // items per segment (a multiple of kSortTile, or n)
-  int blocks_per_segment;
-  int segments;
-};
+constexpr int kDigits = 256, kDigitBits = 8, kPasses = 4;
 
-__global__ void __launch_bounds__(kSortThreads)
-    k_radix_upsweep(const uint32_t* __restrict__ keys, RadixPass p, uint32_t* __restrict__ hist) {
-  __shared__ uint32_t h[kMaxBins];
-  const int bins = 1 << p.bits;
-  for (int d = threadIdx.x; d < bins; d += blockDim.x) h[d] = 0;
+// Digit counts of one tile of kItems x kSortThreads keys.
+template <int kItems>
+__device__ __forceinline__ void tile_histogram(const uint32_t* __restrict__ keys, int shift,
+                                               uint32_t* h) {
+  for (int d = threadIdx.x; d < kDigits; d += kSortThreads) h[d] = 0;
   __syncthreads();
-  const int seg = blockIdx.x / p.blocks_per_segment;
-  const int bis = blockIdx.x % p.blocks_per_segment;
-  const int64_t n = p.n_device != nullptr ? min(*p.n_device, p.n) : p.n;
-  const int64_t seg_begin = (int64_t)seg * p.segment_len;
-  const int64_t seg_end = min(seg_begin + p.segment_len, n);
-  const int64_t begin = seg_begin + (int64_t)bis * kSortTile;
-  const uint32_t mask = (uint32_t)bins - 1u;
-  uint32_t key[kSortItemsPerThread];
+  const int64_t begin = (int64_t)blockIdx.x * (kItems * kSortThreads);
+  uint32_t key[kItems];
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k) {
-    const int64_t i = begin + (int64_t)k * kSortThreads + threadIdx.x;
-    key[k] = i < seg_end ? keys[i] : 0xFFFFFFFFu;
-  }
+  for (int k = 0; k < kItems; ++k) key[k] = keys[begin + k * kSortThreads + threadIdx.x];
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k) {
-    const int64_t i = begin + (int64_t)k * kSortThreads + threadIdx.x;
-    if (i < seg_end) atomicAdd(&h[(key[k] >> p.shift) & mask], 1u);
-  }
+  for (int k = 0; k < kItems; ++k) atomicAdd(&h[(key[k] >> shift) & (kDigits - 1)], 1u);
   __syncthreads();
-  for (int d = threadIdx.x; d < bins; d += blockDim.x)
-    hist[((int64_t)seg * bins + d) * p.blocks_per_segment + bis] = h[d];
 }
 
-// Stable scatter of one block tile. Items are warp-striped (warp w owns
-// [w*512, (w+1)*512), item k of a lane at k*32 + lane) and ranked with
-// __match_any_sync per digit, then offset by earlier warps. The tile is
+// The counts as hist[(segment * digits + digit) * blocks per segment + block], the
+// order in which their exclusive scan gives each block its offsets.
+__global__ void __launch_bounds__(kSortThreads)
+    k_radix_upsweep(const uint32_t* __restrict__ keys, int shift, int blocks_per_segment,
+                    uint32_t* __restrict__ hist) {
+  __shared__ uint32_t h[kDigits];
+  tile_histogram<kSortItemsPerThread>(keys, shift, h);
+  const int seg = blockIdx.x / blocks_per_segment, bis = blockIdx.x % blocks_per_segment;
+  for (int d = threadIdx.x; d < kDigits; d += kSortThreads)
+    hist[((int64_t)seg * kDigits + d) * blocks_per_segment + bis] = h[d];
+}
+
+// For the passes that count as they go (below): the first pass's counts as
+// hist[block * digits + digit], and cleared counts for the other passes.
+template <int kItems>
+__global__ void __launch_bounds__(kSortThreads)
+    k_radix_counts(const uint32_t* __restrict__ keys, uint32_t* __restrict__ hist) {
+  __shared__ uint32_t h[kDigits];
+  tile_histogram<kItems>(keys, 0, h);
+  const int64_t pass_size = (int64_t)gridDim.x * kDigits;
+  for (int d = threadIdx.x; d < kDigits; d += kSortThreads) {
+    uint32_t* at = hist + (int64_t)blockIdx.x * kDigits + d;
+    at[0] = h[d];
+#pragma unroll
+    for (int p = 1; p < kPasses; ++p) at[p * pass_size] = 0;
+  }
+}
+
+// Stable scatter of one block tile by one digit. Items are warp-striped (warp w
+// owns kItems * 32 consecutive ones, item k of a lane at k*32 + lane) and ranked
+// with __match_any_sync per digit, then offset by earlier warps. The tile is
 // reordered by digit in shared memory and written out digit run by digit run,
-// so consecutive threads write consecutive addresses.
+// so consecutive threads write consecutive addresses. vals_in null: the values
+// are the items' places.
+//
+// Where the block's digit runs begin: `offsets` is the scan of k_radix_upsweep's
+// counts, or (kCounting) the counts themselves by block, which each block sums for
+// itself, and each item written also counts towards its tile of the next pass
+// (`next`, null in the last). That spares two launches a pass and is for few
+// enough blocks (depth_sort).
+template <int kItems, bool kCounting>
 __global__ void __launch_bounds__(kSortThreads)
     k_radix_downsweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                       uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
-                      RadixPass p, const uint32_t* __restrict__ offsets) {
+                      int shift, int blocks_per_segment, const uint32_t* __restrict__ offsets,
+                      uint32_t* __restrict__ next) {
+  constexpr int kTileItems = kItems * kSortThreads;
+  constexpr int kStageWords = kTileItems > kSortWarps * kDigits ? kTileItems : kSortWarps * kDigits;
   // per-warp digit counters; reused as the staging buffer once ranks are known
-  __shared__ uint32_t counts[kSortWarps * kMaxBins];
-  __shared__ uint32_t block_offset[kMaxBins];
-  __shared__ uint32_t digit_start[kMaxBins];
+  __shared__ uint32_t counts[kStageWords];
+  __shared__ uint32_t block_offset[kDigits];
+  __shared__ uint32_t digit_start[kDigits];
   __shared__ uint32_t warp_sums[32];
-  static_assert(kSortWarps * kMaxBins >= kSortTile, "staging buffer too small");
-  static_assert(2 * kSortThreads >= kMaxBins, "two digits per thread");
-  const int bins = 1 << p.bits;
-  const uint32_t mask = (uint32_t)bins - 1u;
-  const int seg = blockIdx.x / p.blocks_per_segment;
-  const int bis = blockIdx.x % p.blocks_per_segment;
-  const int64_t n = p.n_device != nullptr ? min(*p.n_device, p.n) : p.n;
-  const int64_t seg_begin = (int64_t)seg * p.segment_len;
-  const int64_t seg_end = min(seg_begin + p.segment_len, n);
-  const int64_t begin = seg_begin + (int64_t)bis * kSortTile;
-  const int64_t end = min(begin + kSortTile, seg_end);
-  const int items = end > begin ? (int)(end - begin) : 0;
-  for (int d = threadIdx.x; d < bins; d += blockDim.x) {
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) counts[w * kMaxBins + d] = 0;
-    block_offset[d] = offsets[((int64_t)seg * bins + d) * p.blocks_per_segment + bis];
-  }
-  __syncthreads();
+  static_assert(kSortThreads == kDigits, "a digit per thread");
+  const int t = threadIdx.x;
+  const int seg = blockIdx.x / blocks_per_segment, bis = blockIdx.x % blocks_per_segment;
+  const int64_t begin = (int64_t)blockIdx.x * kTileItems;
   const int warp = warp_id(), lane = lane_id();
   const unsigned lt = lanemask_lt();
-  uint32_t key[kSortItemsPerThread], val[kSortItemsPerThread], rank[kSortItemsPerThread];
-  int digit[kSortItemsPerThread];
+  uint32_t key[kItems], val[kItems], rank[kItems];
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k) {
-    const int local = warp * (kSortItemsPerThread * 32) + k * 32 + lane;
-    const bool valid = local < items;
-    key[k] = valid ? keys_in[begin + local] : 0u;
-    val[k] = valid ? vals_in[begin + local] : 0u;
-    digit[k] = valid ? (int)((key[k] >> p.shift) & mask) : kMaxBins;  // sentinel groups invalid
+  for (int k = 0; k < kItems; ++k) {
+    const int64_t i = begin + warp * (kItems * 32) + k * 32 + lane;
+    key[k] = keys_in[i];
+    val[k] = vals_in != nullptr ? vals_in[i] : (uint32_t)i;
   }
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k) {
-    const int d = digit[k];
+  for (int w = 0; w < kSortWarps; ++w) counts[w * kDigits + t] = 0;
+  uint32_t before = 0, whole = 0;  // of digit t: in the segment's earlier blocks, in all
+  if (kCounting) {
+    const uint32_t* column = offsets + (int64_t)seg * blocks_per_segment * kDigits + t;
+#pragma unroll 8
+    for (int b = 0; b < blocks_per_segment; ++b) {
+      const uint32_t n = column[(int64_t)b * kDigits];
+      whole += n;
+      before += b < bis ? n : 0u;
+    }
+  } else {
+    block_offset[t] = offsets[((int64_t)seg * kDigits + t) * blocks_per_segment + bis];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kItems; ++k) {
+    const uint32_t d = (key[k] >> shift) & (kDigits - 1);
     const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0;
-    if (d < kMaxBins) base = counts[warp * kMaxBins + d];
+    const uint32_t base = counts[warp * kDigits + d];
     __syncwarp();
-    if (lane == leader && d < kMaxBins) counts[warp * kMaxBins + d] = base + __popc(peers);
+    if (lane == __ffs(peers) - 1) counts[warp * kDigits + d] = base + __popc(peers);
     __syncwarp();
     rank[k] = base + __popc(peers & lt);
   }
   __syncthreads();
-  // thread t owns digits 2t and 2t+1: exclusive prefix over warps in place,
-  // then the block-local start of each digit by a scan in digit order
-  uint32_t total_pair[2] = {0u, 0u};
+  // digit t: exclusive prefix over warps in place, then the block-local start of
+  // each digit by a scan in digit order
+  uint32_t run = 0;
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int d = 2 * (int)threadIdx.x + r;
-    if (d < bins) {
-      uint32_t run = 0;
-#pragma unroll
-      for (int w = 0; w < kSortWarps; ++w) {
-        const uint32_t c = counts[w * kMaxBins + d];
-        counts[w * kMaxBins + d] = run;
-        run += c;
-      }
-      total_pair[r] = run;
-    }
+  for (int w = 0; w < kSortWarps; ++w) {
+    const uint32_t c = counts[w * kDigits + t];
+    counts[w * kDigits + t] = run;
+    run += c;
   }
   uint32_t block_total;
-  const uint32_t start = block_exclusive_scan<uint32_t>(total_pair[0] + total_pair[1],
-                                                         &block_total, warp_sums);
-  if (2 * (int)threadIdx.x < bins) digit_start[2 * threadIdx.x] = start;
-  if (2 * (int)threadIdx.x + 1 < bins) digit_start[2 * threadIdx.x + 1] = start + total_pair[0];
+  digit_start[t] = block_exclusive_scan<uint32_t>(run, &block_total, warp_sums);
+  if (kCounting)
+    block_offset[t] = (uint32_t)seg * blocks_per_segment * kTileItems + before +
+                      block_exclusive_scan<uint32_t>(whole, &block_total, warp_sums);
   __syncthreads();
-  uint32_t local_pos[kSortItemsPerThread];
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k) {
-    const int d = digit[k];
-    local_pos[k] = d < kMaxBins ? digit_start[d] + counts[warp * kMaxBins + d] + rank[k] : 0u;
+  for (int k = 0; k < kItems; ++k) {
+    const uint32_t d = (key[k] >> shift) & (kDigits - 1);
+    rank[k] += digit_start[d] + counts[warp * kDigits + d];  // the place in the tile
   }
   __syncthreads();  // counts is now free: stage the keys by digit
-  uint32_t* stage = counts;
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k)
-    if (digit[k] < kMaxBins) stage[local_pos[k]] = key[k];
+  for (int k = 0; k < kItems; ++k) counts[rank[k]] = key[k];
   __syncthreads();
-  uint32_t global_pos[kSortItemsPerThread];
+  uint32_t to[kItems];
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k) {
-    const int i = k * kSortThreads + threadIdx.x;
-    global_pos[k] = 0xFFFFFFFFu;
-    if (i < items) {
-      const uint32_t kk = stage[i];
-      const int d = (int)((kk >> p.shift) & mask);
-      global_pos[k] = block_offset[d] + ((uint32_t)i - digit_start[d]);
-      keys_out[global_pos[k]] = kk;
-    }
+  for (int k = 0; k < kItems; ++k) {
+    const int i = k * kSortThreads + t;
+    const uint32_t kk = counts[i];
+    const uint32_t d = (kk >> shift) & (kDigits - 1);
+    to[k] = block_offset[d] + ((uint32_t)i - digit_start[d]);
+    keys_out[to[k]] = kk;
+    if (kCounting && next != nullptr)
+      atomicAdd(&next[(int64_t)(to[k] / kTileItems) * kDigits +
+                      ((kk >> (shift + kDigitBits)) & (kDigits - 1))],
+                1u);
   }
   __syncthreads();  // stage the values the same way
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k)
-    if (digit[k] < kMaxBins) stage[local_pos[k]] = val[k];
+  for (int k = 0; k < kItems; ++k) counts[rank[k]] = val[k];
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < kSortItemsPerThread; ++k) {
-    const int i = k * kSortThreads + threadIdx.x;
-    if (i < items) vals_out[global_pos[k]] = stage[i];
-  }
+  for (int k = 0; k < kItems; ++k) vals_out[to[k]] = counts[k * kSortThreads + t];
 }
-
-__global__ void k_iota(uint32_t* __restrict__ out, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = (uint32_t)i;
-}
-
 
 }  // namespace
 
@@ -308,51 +300,74 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, ScanScratc
   scan_impl<uint32_t, uint32_t>(in, out, n, nullptr, scratch, 0, stream);
 }
 
-size_t radix_hist_entries(int64_t n, int64_t segment_len, int max_bits) {
-  const int64_t seg_len = segment_len > 0 ? segment_len : n;
-  const int segments = (int)((n + seg_len - 1) / seg_len);
-  const int bps = (int)((seg_len + kSortTile - 1) / kSortTile);
-  return (size_t)segments * ((size_t)1 << max_bits) * (size_t)bps;
+namespace {
+
+// Items per thread of the counting passes, 0 where they do not pay: their blocks
+// each sum every block's counts of their view (up to 128 loads per thread) and
+// count each item with a global atomic, but a sort is 5 launches instead of 12 to
+// 20, and small tiles spread a small cloud over the SMs. The binning stage in us,
+// with and without: 60 / 78 (4k slots), 68 / 87 (20k), 90 / 126 (3 x 40k), 93 / 120
+// (60k), 124 / 131 (152k; 131 with 16 items), 173 / 184 (300k), 150 / 147 (400k).
+int counting_items(int64_t segment_len, int64_t n) {
+  if (n > (int64_t)1 << 20 || segment_len > (int64_t)3 << 17) return 0;
+  return segment_len <= (int64_t)1 << 16 ? 4 : segment_len <= (int64_t)1 << 18 ? 8 : 16;
 }
 
-int radix_sort_pairs(uint32_t*& keys, uint32_t*& vals, uint32_t*& keys_alt,
-                     uint32_t*& vals_alt, int64_t n, int64_t segment_len, int total_bits,
-                     uint32_t* hist, uint32_t* hist_scanned, ScanScratch& scratch,
-                     cudaStream_t stream, const int64_t* n_device) {
-  if (n <= 0 || total_bits <= 0) return 0;
-  const int64_t seg_len = segment_len > 0 ? segment_len : n;
-  const int passes = (total_bits + 8) / 9 > 0 ? (total_bits + 8) / 9 : 1;
-  RadixPass p;
-  p.n = n;
-  p.n_device = n_device;
-  p.segment_len = seg_len;
-  p.segments = (int)((n + seg_len - 1) / seg_len);
-  p.blocks_per_segment = (int)((seg_len + kSortTile - 1) / kSortTile);
-  const int blocks = p.segments * p.blocks_per_segment;
-  int shift = 0;
-  for (int pass = 0; pass < passes; ++pass) {
-    const int remaining = total_bits - shift;
-    const int bits = (remaining + (passes - pass) - 1) / (passes - pass);
-    p.shift = shift;
-    p.bits = bits;
+template <int kItems>
+void counting_sort(const uint32_t* keys, int64_t n, int64_t segment_len, uint32_t* keys_a,
+                   uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, uint32_t* hist,
+                   cudaStream_t stream) {
+  const int tile = kItems * kSortThreads;
+  const int blocks = (int)(n / tile), per_segment = (int)(segment_len / tile);
+  const int64_t pass_size = (int64_t)blocks * kDigits;
+  count_launch();
+  k_radix_counts<kItems><<<blocks, kSortThreads, 0, stream>>>(keys, hist);
+  const uint32_t *ki = keys, *vi = nullptr;
+  for (int p = 0; p < kPasses; ++p) {
+    uint32_t *ko = p % 2 ? keys_b : keys_a, *vo = p % 2 ? vals_b : vals_a;
     count_launch();
-    k_radix_upsweep<<<blocks, kSortThreads, 0, stream>>>(keys, p, hist);
-    const int64_t entries = (int64_t)p.segments * ((int64_t)1 << bits) * p.blocks_per_segment;
-    exclusive_scan_u32(hist, hist_scanned, entries, scratch, stream);
-    count_launch();
-    k_radix_downsweep<<<blocks, kSortThreads, 0, stream>>>(keys, vals, keys_alt, vals_alt, p,
-                                                           hist_scanned);
-    std::swap(keys, keys_alt);
-    std::swap(vals, vals_alt);
-    shift += bits;
+    k_radix_downsweep<kItems, true><<<blocks, kSortThreads, 0, stream>>>(
+        ki, vi, ko, vo, p * kDigitBits, per_segment, hist + p * pass_size,
+        p + 1 < kPasses ? hist + (p + 1) * pass_size : nullptr);
+    ki = ko;
+    vi = vo;
   }
-  return passes;
 }
 
-void launch_iota(uint32_t* out, int64_t n, cudaStream_t stream) {
-  if (n > 0) {
-    count_launch();
-    k_iota<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(out, n);
+}  // namespace
+
+size_t depth_sort_hist_entries(int64_t n, int64_t segment_len) {
+  const int items = counting_items(segment_len, n);
+  return items > 0 ? (size_t)(n / (items * kSortThreads)) * kDigits * kPasses
+                   : (size_t)(n / kSortTile) * kDigits;
+}
+
+void depth_sort(const uint32_t* keys, int64_t n, int64_t segment_len, uint32_t* keys_a,
+                uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, uint32_t* hist,
+                uint32_t* hist_scanned, ScanScratch& scratch, cudaStream_t stream) {
+  static_assert(kPasses % 2 == 0, "the result lies in the b buffers");
+  if (n <= 0) return;
+  const int items = counting_items(segment_len, n);
+  if (items == 4) {
+    counting_sort<4>(keys, n, segment_len, keys_a, vals_a, keys_b, vals_b, hist, stream);
+  } else if (items == 8) {
+    counting_sort<8>(keys, n, segment_len, keys_a, vals_a, keys_b, vals_b, hist, stream);
+  } else if (items == 16) {
+    counting_sort<16>(keys, n, segment_len, keys_a, vals_a, keys_b, vals_b, hist, stream);
+  } else {
+    const int blocks = (int)(n / kSortTile), per_segment = (int)(segment_len / kSortTile);
+    const uint32_t *ki = keys, *vi = nullptr;
+    for (int p = 0; p < kPasses; ++p) {
+      uint32_t *ko = p % 2 ? keys_b : keys_a, *vo = p % 2 ? vals_b : vals_a;
+      count_launch();
+      k_radix_upsweep<<<blocks, kSortThreads, 0, stream>>>(ki, p * kDigitBits, per_segment, hist);
+      exclusive_scan_u32(hist, hist_scanned, (int64_t)blocks * kDigits, scratch, stream);
+      count_launch();
+      k_radix_downsweep<kSortItemsPerThread, false><<<blocks, kSortThreads, 0, stream>>>(
+          ki, vi, ko, vo, p * kDigitBits, per_segment, hist_scanned, nullptr);
+      ki = ko;
+      vi = vo;
+    }
   }
 }
 

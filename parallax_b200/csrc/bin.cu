@@ -33,6 +33,8 @@
 // With 8 views of 1M gaussians at 1920x1440 binning went from 2.76 to 2.38 ms,
 // compositing, which stages the entries, from 2.63 to 2.27, its adjoint from
 // 4.70 to 4.60.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "raster_common.cuh"
@@ -619,6 +621,164 @@ __global__ void k_row_ranges_from_chunks(const int64_t* __restrict__ offsets, in
   row_ranges[r] = make_int2((int)b, (int)e);
 }
 
+// ------------------------------------------------------- small images, directly
+//
+// With few tiles a view's tiles fit a CTA's shared memory and the lists need no
+// rows in between. A CTA takes 256 depth-sorted slots, one per thread, and keeps a
+// 256-bit map per tile of the ones that reach it: its counts per tile give, summed
+// over the earlier chunks and scanned over the tiles, the chunk's base in every
+// list, and a slot's place from there is the number of earlier bits. 4 launches
+// instead of 9 to 13 (Frame::direct_lists has the times).
+constexpr int kDirectSlots = kWarps * 32;
+
+// The tiles that the thread's slot reaches, f(tile) in row order; `i` its place
+// among the depth-sorted slots.
+struct DirectSlot {
+  uint32_t slot, yr;
+  RowShape shape;
+};
+__device__ __forceinline__ DirectSlot direct_slot(const uint32_t* __restrict__ sorted_slots,
+                                                  const uint32_t* __restrict__ sorted_keys,
+                                                  const SlotGeom* __restrict__ geom, bool tight,
+                                                  float min_alpha, int64_t i) {
+  DirectSlot d;
+  d.slot = sorted_slots[i];
+  d.yr = d.shape.x = 1u;  // 1 > 0: no rows, no columns
+  d.shape.ia = 0.f;
+  if (sorted_keys[i] == kCulledKey) return d;
+  const SlotGeom g = geom[d.slot];
+  d.yr = g.rect.y;
+  d.shape.x = g.rect.x;
+  if (tight && (d.yr >> 16) >= (d.yr & 0xFFFF))
+    d.shape = row_shape(splat_footprint(g.conic_op, min_alpha), g.conic_op, g.xy, g.rect.x);
+  return d;
+}
+template <typename F>
+__device__ __forceinline__ void for_each_reached_tile(const DirectSlot& d, int tiles_x, F&& f) {
+  const int y1 = d.yr >> 16;
+  for (int y = d.yr & 0xFFFF; y <= y1; ++y) {
+    const uint32_t x = row_columns(d.shape, y);
+    const int x1 = x >> 16;
+    for (int c = x & 0xFFFF; c <= x1; ++c) f(y * tiles_x + c);
+  }
+}
+
+// Each warp's bits of the chunk's map, map[kWarps][tiles].
+__device__ __forceinline__ void map_tiles(const DirectSlot& d, int tiles, int tiles_x,
+                                          uint32_t* map) {
+  for (int i = threadIdx.x; i < kWarps * tiles; i += blockDim.x) map[i] = 0u;
+  __syncthreads();
+  uint32_t* mine = map + warp_id() * tiles;
+  const uint32_t bit = 1u << lane_id();
+  for_each_reached_tile(d, tiles_x, [&](int t) { atomicOr(&mine[t], bit); });
+  __syncthreads();
+}
+
+// counts[chunk * total_tiles + tile]: slots of the chunk that reach the tile; a
+// chunk counts its own view's tiles.
+__global__ void __launch_bounds__(kDirectSlots)
+    k_direct_counts(const uint32_t* __restrict__ sorted_slots,
+                    const uint32_t* __restrict__ sorted_keys,
+                    const SlotGeom* __restrict__ geom, int tight,
+                    const ViewDesc* __restrict__ views, int64_t slot_stride, int cpv,
+                    int total_tiles, int32_t* __restrict__ counts) {
+  extern __shared__ uint32_t s_map[];
+  const int v = blockIdx.x / cpv, c = blockIdx.x % cpv;
+  const ViewDesc& vd = views[v];
+  const int tiles = vd.tiles_x * vd.tiles_y;
+  const DirectSlot d = direct_slot(sorted_slots, sorted_keys, geom, tight, vd.min_alpha,
+                                   (int64_t)v * slot_stride + c * kDirectSlots + threadIdx.x);
+  map_tiles(d, tiles, vd.tiles_x, s_map);
+  for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
+    int total = 0;
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) total += __popc(s_map[k * tiles + t]);
+    counts[(int64_t)c * total_tiles + vd.tile_offset + t] = total;
+  }
+}
+
+// The counts become each chunk's base within its tile's list, and the lists'
+// lengths go to tile_counts. 32 tiles per CTA, each warp a range of the chunks.
+__global__ void __launch_bounds__(kWarps * 32)
+    k_direct_bases(int32_t* __restrict__ counts, int cpv, int total_tiles,
+                   int32_t* __restrict__ tile_counts, int32_t* __restrict__ overflow) {
+  __shared__ int s_sum[kWarps][32];
+  const int w = warp_id(), lane = lane_id();
+  const int tile = blockIdx.x * 32 + lane;
+  const int per = (cpv + kWarps - 1) / kWarps;
+  const int c0 = min(cpv, w * per), c1 = min(cpv, c0 + per);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *overflow = 0;
+  int sum = 0;
+  if (tile < total_tiles)
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) sum += counts[(int64_t)c * total_tiles + tile];
+  s_sum[w][lane] = sum;
+  __syncthreads();
+  if (tile >= total_tiles) return;
+  int run = 0;
+  for (int k = 0; k < w; ++k) run += s_sum[k][lane];
+  if (w == kWarps - 1) tile_counts[tile] = run + sum;
+#pragma unroll 4
+  for (int c = c0; c < c1; ++c) {
+    int32_t* at = &counts[(int64_t)c * total_tiles + tile];
+    const int n = *at;
+    *at = run;
+    run += n;
+  }
+}
+
+// The lists; nothing at or past `capacity`. A view's first chunk also writes its
+// tiles' ranges (a tile whose list would pass the capacity is left empty and
+// raises the overflow flag).
+__global__ void __launch_bounds__(kDirectSlots)
+    k_direct_expand(const uint32_t* __restrict__ sorted_slots,
+                    const uint32_t* __restrict__ sorted_keys,
+                    const SlotGeom* __restrict__ geom, int tight,
+                    const ViewDesc* __restrict__ views, int64_t slot_stride, int cpv,
+                    int total_tiles, const int32_t* __restrict__ bases,
+                    const int64_t* __restrict__ tile_offsets,
+                    const int32_t* __restrict__ tile_counts, int64_t capacity,
+                    uint32_t* __restrict__ tile_slots, int2* __restrict__ ranges,
+                    int32_t* __restrict__ overflow) {
+  // per tile: the map, a byte per warp counting the earlier warps' bits, the base
+  extern __shared__ __align__(8) uint32_t s_map[];
+  const int v = blockIdx.x / cpv, c = blockIdx.x % cpv;
+  const ViewDesc& vd = views[v];
+  const int tiles = vd.tiles_x * vd.tiles_y;
+  uint8_t* const before = reinterpret_cast<uint8_t*>(s_map + kWarps * tiles);
+  uint32_t* const base = s_map + (kWarps + 2) * tiles;
+  const DirectSlot d = direct_slot(sorted_slots, sorted_keys, geom, tight, vd.min_alpha,
+                                   (int64_t)v * slot_stride + c * kDirectSlots + threadIdx.x);
+  map_tiles(d, tiles, vd.tiles_x, s_map);
+  for (int t = threadIdx.x; t < tiles; t += blockDim.x) {
+    const int64_t tile = vd.tile_offset + t;
+    const int64_t first = tile_offsets[tile];
+    // list positions in 32 bits: nothing past the capacity is written
+    base[t] = (uint32_t)min(first + bases[(int64_t)c * total_tiles + tile], capacity);
+    uint64_t packed = 0;
+    int run = 0;  // at most 7 * 32 before the last warp
+#pragma unroll
+    for (int k = 0; k < kWarps; ++k) {
+      packed |= (uint64_t)run << (8 * k);
+      run += __popc(s_map[k * tiles + t]);
+    }
+    reinterpret_cast<uint64_t*>(before)[t] = packed;
+    if (c == 0) {
+      const int64_t end = first + tile_counts[tile];
+      ranges[tile] = end <= capacity ? make_int2((int)first, (int)end) : make_int2(0, 0);
+      if (end > capacity) atomicExch(overflow, 1);
+    }
+  }
+  __syncthreads();
+  const int w = warp_id();
+  const uint32_t* mine = s_map + w * tiles;
+  const unsigned lt = lanemask_lt();
+  for_each_reached_tile(d, vd.tiles_x, [&](int t) {
+    const uint64_t at = (uint64_t)base[t] + before[8 * t + w] + __popc(mine[t] & lt);
+    if (at < (uint64_t)capacity) tile_slots[at] = d.slot;
+  });
+}
+
 // ------------------------------------------------------------------ host
 
 size_t chunk_counts_smem(int max_tiles_x) { return sizeof(int32_t) * kWarps * max_tiles_x; }
@@ -631,9 +791,16 @@ size_t slot_row_expand_smem(int max_tiles_y) {
   return sizeof(RowExpandSmem) + chunk_expand_smem(max_tiles_y) - sizeof(int32_t) * kStage;
 }
 
+size_t direct_counts_smem(int tiles) { return sizeof(uint32_t) * kWarps * (size_t)tiles; }
+size_t direct_expand_smem(int tiles) { return sizeof(uint32_t) * (kWarps + 3) * (size_t)tiles; }
+
 size_t slot_row_counts_smem(int max_tiles_y) { return sizeof(int32_t) * kWarps * max_tiles_y; }
 
 void configure_bin_kernels() {
+  cudaFuncSetAttribute(k_direct_counts, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)direct_counts_smem(kMaxDirectTiles));
+  cudaFuncSetAttribute(k_direct_expand, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)direct_expand_smem(kMaxDirectTiles));
   cudaFuncSetAttribute(k_chunk_counts, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)chunk_counts_smem(kMaxTilesX));
   cudaFuncSetAttribute(k_chunk_expand, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -679,6 +846,36 @@ void launch_row_ranges_from_chunks(const int64_t* offsets, int total_rows, int c
   count_launch();
   k_row_ranges_from_chunks<<<(unsigned)((total_rows + 255) / 256), 256, 0, stream>>>(
       offsets, total_rows, cpv, total, capacity, row_ranges, overflow);
+}
+
+int direct_chunks_per_view(int64_t slot_stride) { return (int)(slot_stride / kDirectSlots); }
+
+void launch_direct_counts(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
+                          const SlotGeom* geom, bool tight, const ViewDesc* views, int n_views,
+                          int64_t slot_stride, int max_tiles, int total_tiles, int32_t* counts,
+                          int32_t* tile_counts, int32_t* overflow, cudaStream_t stream) {
+  const int cpv = direct_chunks_per_view(slot_stride);
+  count_launch();
+  k_direct_counts<<<(unsigned)(n_views * cpv), kDirectSlots, direct_counts_smem(max_tiles),
+                    stream>>>(sorted_slots, sorted_keys, geom, tight, views, slot_stride, cpv,
+                              total_tiles, counts);
+  count_launch();
+  k_direct_bases<<<(unsigned)std::max(1, (total_tiles + 31) / 32), kWarps * 32, 0, stream>>>(
+      counts, cpv, total_tiles, tile_counts, overflow);
+}
+
+void launch_direct_expand(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
+                          const SlotGeom* geom, bool tight, const ViewDesc* views, int n_views,
+                          int64_t slot_stride, int max_tiles, int total_tiles,
+                          const int32_t* bases, const int64_t* tile_offsets,
+                          const int32_t* tile_counts, int64_t capacity, uint32_t* tile_slots,
+                          int2* ranges, int32_t* overflow, cudaStream_t stream) {
+  const int cpv = direct_chunks_per_view(slot_stride);
+  count_launch();
+  k_direct_expand<<<(unsigned)(n_views * cpv), kDirectSlots, direct_expand_smem(max_tiles),
+                    stream>>>(sorted_slots, sorted_keys, geom, tight, views, slot_stride, cpv,
+                              total_tiles, bases, tile_offsets, tile_counts, capacity,
+                              tile_slots, ranges, overflow);
 }
 
 int64_t max_row_chunks(int64_t records, int total_rows) { return records / kChunk + total_rows + 1; }

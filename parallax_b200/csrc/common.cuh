@@ -25,6 +25,9 @@ constexpr uint32_t kCulledKey = 0xFFFFFFFFu;
 // Widest image, in tiles, the row-binning kernels stage in shared memory.
 constexpr int kMaxTilesX = 2048;
 constexpr int kMaxTilesY = 2048;
+// Most tiles of a view whose lists are built directly, without tile rows
+// (Frame::direct_lists).
+constexpr int kMaxDirectTiles = 2048;
 
 // Everything a kernel needs to know about one view of a batch.
 struct ViewDesc {

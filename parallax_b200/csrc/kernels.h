@@ -80,6 +80,21 @@ void launch_slot_row_expand(const uint32_t* sorted_slots, const uint32_t* sorted
 void launch_row_ranges_from_chunks(const int64_t* offsets, int total_rows, int cpv,
                                    const int64_t* total, int64_t capacity, int2* row_ranges,
                                    int32_t* overflow, cudaStream_t stream);
+// The tile lists of views of few tiles (at most kMaxDirectTiles each) directly:
+// counts [chunks of a view][total_tiles] become the chunks' bases within their
+// tiles' lists, tile_counts the lists' lengths (overflow is cleared); after the
+// lengths' scan into tile_offsets the lists and ranges.
+int direct_chunks_per_view(int64_t slot_stride);
+void launch_direct_counts(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
+                          const SlotGeom* geom, bool tight, const ViewDesc* views, int n_views,
+                          int64_t slot_stride, int max_tiles, int total_tiles, int32_t* counts,
+                          int32_t* tile_counts, int32_t* overflow, cudaStream_t stream);
+void launch_direct_expand(const uint32_t* sorted_slots, const uint32_t* sorted_keys,
+                          const SlotGeom* geom, bool tight, const ViewDesc* views, int n_views,
+                          int64_t slot_stride, int max_tiles, int total_tiles,
+                          const int32_t* bases, const int64_t* tile_offsets,
+                          const int32_t* tile_counts, int64_t capacity, uint32_t* tile_slots,
+                          int2* ranges, int32_t* overflow, cudaStream_t stream);
 // Upper bound on the number of row chunks for `records` records.
 int64_t max_row_chunks(int64_t records, int total_rows);
 // Chunk table, per-chunk column counts, per-chunk bases and tile lengths.

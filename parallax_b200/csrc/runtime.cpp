@@ -73,6 +73,7 @@ ViewBatch make_batch(const pxs_camera* cameras, int n_views, const pxs_raster_op
     row_offset += d.tiles_y;
     b.max_tiles_x = std::max(b.max_tiles_x, d.tiles_x);
     b.max_tiles_y = std::max(b.max_tiles_y, d.tiles_y);
+    b.max_tiles = std::max(b.max_tiles, d.tiles_x * d.tiles_y);
     pixel_offset += static_cast<int64_t>(d.cam.width) * d.cam.height;
   }
   std::vector<int> widths, heights;
@@ -137,8 +138,10 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   sort_vals.reserve(slots);
   sort_keys_alt.reserve(slots);
   sort_vals_alt.reserve(slots);
-  const size_t row_chunks = static_cast<size_t>(std::max(batch.total_rows, 1)) *
-                            static_cast<size_t>(std::max(slot_chunks_per_view(slot_stride), 1));
+  const size_t row_chunks =
+      direct_lists()
+          ? static_cast<size_t>(std::max(batch.total_tiles, 1)) * direct_chunks_per_view(slot_stride)
+          : static_cast<size_t>(std::max(batch.total_rows, 1)) * slot_chunks_per_view(slot_stride);
   row_chunk_counts.reserve(row_chunks);
   row_chunk_offsets.reserve(row_chunks);
   d_total_pairs.reserve(1);
@@ -169,7 +172,8 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   }
   ensure_scan_scratch(std::max<int64_t>(std::max<int64_t>(static_cast<int64_t>(slots),
                                                           static_cast<int64_t>(hist.capacity())),
-                                        batch.total_tiles));
+                                        static_cast<int64_t>(
+                                            std::max<size_t>(row_chunks, batch.total_tiles))));
   // the chunk table depends on the rows as well as on the record capacity; size
   // it here, before any stream capture of the binning stage
   if (record_capacity > 0) ensure_chunks();
@@ -218,6 +222,19 @@ void Frame::project(const float* params, cudaStream_t stream, bool want_debug,
   PXS_CUDA(cudaGetLastError());
 }
 
+// The direct lists keep a map over a view's tiles in shared memory, and clear and
+// read it once per 256 slots: their time grows with tiles times slots, that of the
+// lists by rows with the records. The binning stage in us, directly / by rows: 37 /
+// 58 (4k slots, 64 tiles), 47 / 68 (20k, 300), 68 / 91 (3 views of 38k, 1080), 76 /
+// 93 (60k, 1938), 86 / 105 (150k, 1200), 168 / 221 (8 views of 150k, 300 tiles: 1.4M
+// counts); past the line 131 / 119 (200k, 1900), 171 / 156 (400k, 1200), 272 / 197
+// (8 of 100k, 1900), and 228 / 213 (800k, 300) for the slots alone.
+bool Frame::direct_lists() const {
+  return batch.max_tiles <= kMaxDirectTiles && slot_stride <= (1 << 18) &&
+         static_cast<int64_t>(batch.total_tiles) * direct_chunks_per_view(slot_stride) <=
+             1450000;
+}
+
 int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
   order_ready = false;  // new tile lists
   const int64_t slots = static_cast<int64_t>(V) * slot_stride;
@@ -231,6 +248,34 @@ int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
   const uint32_t* const k = sort_keys.get();  // kCulledKey for a culled slot
   uint32_t* const v = sort_vals.get();
   sorted_slots = v;
+  if (direct_lists()) {
+    launch_direct_counts(v, k, geom.get(), !whole_lists_, d_views.get(), V, slot_stride,
+                         batch.max_tiles, batch.total_tiles, row_chunk_counts.get(),
+                         tile_counts.get(), overflow.get(), stream);
+    exclusive_scan_i32_to_i64(tile_counts.get(), tile_offsets.get(), batch.total_tiles,
+                              d_total_pairs.get(), scan_, stream);
+    PXS_CUDA(cudaGetLastError());
+    last_record_count = 0;
+    if (host_sync) {
+      PXS_CUDA(cudaMemcpyAsync(&last_pair_count, d_total_pairs.get(), sizeof(int64_t),
+                               cudaMemcpyDeviceToHost, stream));
+      PXS_CUDA(cudaStreamSynchronize(stream));
+      if (last_pair_count > pair_capacity)
+        reserve_pairs(last_pair_count + last_pair_count / 8 + 1024);
+    }
+    if (tile_slots.get() == nullptr) {
+      if (!host_sync)
+        throw Error(PXS_ERR_INVALID, "pair buffers must be reserved before an unsynchronised bin");
+      reserve_pairs(1024);
+    }
+    launch_direct_expand(v, k, geom.get(), !whole_lists_, d_views.get(), V, slot_stride,
+                         batch.max_tiles, batch.total_tiles, row_chunk_counts.get(),
+                         tile_offsets.get(), tile_counts.get(), pair_capacity, tile_slots.get(),
+                         ranges.get(), overflow.get(), stream);
+    sorted_pair_vals = tile_slots.get();
+    PXS_CUDA(cudaGetLastError());
+    return host_sync ? last_pair_count : -1;
+  }
   // 2. one record per covered tile row, grouped by row and near to far within
   //    a row: per (view, slot chunk) row counts, their scan in (row, chunk)
   //    order, then each chunk writes its records at its bases

@@ -93,6 +93,7 @@ struct ViewBatch {
   int total_tiles = 0;
   int total_rows = 0;       // tile rows over all views
   int max_tiles_x = 0, max_tiles_y = 0;
+  int max_tiles = 0;        // of one view
   int loss_rows = 0;        // output rows per CTA of the loss
   int64_t loss_blocks = 0, l1_blocks = 0;
   // the views carry their own gaussian ranges (several scenes); otherwise
@@ -193,6 +194,8 @@ class Frame {
 
  private:
   bool whole_lists_ = false;
+  // Whether the tile lists are built directly (bin.cu).
+  bool direct_lists() const;
   void ensure_scan_scratch(int64_t n);
   void ensure_chunks();
   ScanScratch scan_;

@@ -75,11 +75,6 @@ void launch_slot_row_expand(const uint32_t* sorted_slots, const uint32_t* sorted
                             int64_t slot_stride, int max_tiles_y, const int64_t* offsets,
                             int64_t capacity, uint32_t* rec_slots, uint32_t* rec_xr,
                             cudaStream_t stream);
-// Per-row record ranges from the chunk offsets, clamped to the capacity
-// (records past it raise the overflow flag).
-void launch_row_ranges_from_chunks(const int64_t* offsets, int total_rows, int cpv,
-                                   const int64_t* total, int64_t capacity, int2* row_ranges,
-                                   int32_t* overflow, cudaStream_t stream);
 // The tile lists of views of few tiles (at most kMaxDirectTiles each) directly:
 // counts [chunks of a view][total_tiles] become the chunks' bases within their
 // tiles' lists, tile_counts the lists' lengths (overflow is cleared); after the
@@ -97,12 +92,15 @@ void launch_direct_expand(const uint32_t* sorted_slots, const uint32_t* sorted_k
                           int2* ranges, int32_t* overflow, cudaStream_t stream);
 // Upper bound on the number of row chunks for `records` records.
 int64_t max_row_chunks(int64_t records, int total_rows);
-// Chunk table, per-chunk column counts, per-chunk bases and tile lengths.
-void launch_tile_lists(const int2* row_ranges, const uint32_t* rec_slots, const uint32_t* rec_xr,
-                       const ViewDesc* views, int n_views, int total_rows, int max_tiles_x,
-                       int64_t max_chunks, int4* chunks, int32_t* n_chunks,
-                       int32_t* chunk_counts, int32_t* chunk_base, int32_t* tile_counts,
-                       cudaStream_t stream);
+// Chunk table (from the records' offsets by row and slot chunk, as
+// launch_slot_row_expand took them; records past the capacity raise the overflow
+// flag), per-chunk column counts, per-chunk bases and tile lengths.
+void launch_tile_lists(const int64_t* offsets, int cpv, const int64_t* total_records,
+                       int64_t record_capacity, const uint32_t* rec_slots,
+                       const uint32_t* rec_xr, const ViewDesc* views, int n_views,
+                       int total_rows, int max_tiles_x, int64_t max_chunks, int4* chunks,
+                       int32_t* n_chunks, int32_t* chunk_counts, int32_t* chunk_base,
+                       int32_t* tile_counts, int32_t* overflow, cudaStream_t stream);
 void launch_ranges_from_offsets(const int32_t* counts, const int64_t* offsets, int64_t n_tiles,
                                 int64_t capacity, int2* ranges, int32_t* overflow,
                                 cudaStream_t stream);

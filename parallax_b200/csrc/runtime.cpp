@@ -159,7 +159,6 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   order_ready = false;
   tile_counts.reserve(static_cast<size_t>(std::max(batch.total_tiles, 1)));
   tile_offsets.reserve(static_cast<size_t>(std::max(batch.total_tiles, 1)));
-  row_ranges.reserve(static_cast<size_t>(std::max(batch.total_rows, 1)));
   n_chunks.reserve(1);
   d_total_records.reserve(1);
   loss_sums.reserve(static_cast<size_t>(2 * std::max(V, 1) + 1));
@@ -299,15 +298,13 @@ int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
   launch_slot_row_expand(v, k, geom.get(), !whole_lists_, d_views.get(), V, slot_stride,
                          batch.max_tiles_y, row_chunk_offsets.get(), record_capacity,
                          rec_vals.get(), rec_xr.get(), stream);
-  launch_row_ranges_from_chunks(row_chunk_offsets.get(), batch.total_rows, cpv,
-                                d_total_records.get(), record_capacity, row_ranges.get(),
-                                overflow.get(), stream);
   const uint32_t* rv = rec_vals.get();
   // 4. tile lengths from chunked rows, their offsets, then the lists themselves
   ensure_chunks();
-  launch_tile_lists(row_ranges.get(), rv, rec_xr.get(), d_views.get(), V, batch.total_rows,
-                    batch.max_tiles_x, max_chunks, chunks.get(), n_chunks.get(),
-                    chunk_counts.get(), chunk_base.get(), tile_counts.get(), stream);
+  launch_tile_lists(row_chunk_offsets.get(), cpv, d_total_records.get(), record_capacity, rv,
+                    rec_xr.get(), d_views.get(), V, batch.total_rows, batch.max_tiles_x,
+                    max_chunks, chunks.get(), n_chunks.get(), chunk_counts.get(),
+                    chunk_base.get(), tile_counts.get(), overflow.get(), stream);
   exclusive_scan_i32_to_i64(tile_counts.get(), tile_offsets.get(), batch.total_tiles,
                             d_total_pairs.get(), scan_, stream);
   PXS_CUDA(cudaGetLastError());

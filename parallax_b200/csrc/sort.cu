@@ -189,6 +189,9 @@ __global__ void __launch_bounds__(kSortThreads)
   __shared__ uint32_t block_offset[kDigits];
   __shared__ uint32_t digit_start[kDigits];
   __shared__ uint32_t warp_sums[32];
+  // of each digit, by fourth block: in the segment's blocks, in the earlier ones
+  __shared__ __align__(16) uint32_t s_whole[kCounting ? 4 : 1][kCounting ? kDigits : 4];
+  __shared__ __align__(16) uint32_t s_before[kCounting ? 4 : 1][kCounting ? kDigits : 4];
   static_assert(kSortThreads == kDigits, "a digit per thread");
   const int t = threadIdx.x;
   const int seg = blockIdx.x / blocks_per_segment, bis = blockIdx.x % blocks_per_segment;
@@ -204,15 +207,30 @@ __global__ void __launch_bounds__(kSortThreads)
   }
 #pragma unroll
   for (int w = 0; w < kSortWarps; ++w) counts[w * kDigits + t] = 0;
-  uint32_t before = 0, whole = 0;  // of digit t: in the segment's earlier blocks, in all
   if (kCounting) {
-    const uint32_t* column = offsets + (int64_t)seg * blocks_per_segment * kDigits + t;
+    // a quarter of the threads per fourth block, four digits per thread: the
+    // segment's counts in a few rounds of 16-byte loads (one digit per thread
+    // took a round per eight blocks, most of the kernel at 74 blocks)
+    const uint4* rows = reinterpret_cast<const uint4*>(
+        offsets + (int64_t)seg * blocks_per_segment * kDigits);
+    const int phase = t >> 6, quad = t & 63;
+    uint4 whole = make_uint4(0, 0, 0, 0), before = whole;
 #pragma unroll 8
-    for (int b = 0; b < blocks_per_segment; ++b) {
-      const uint32_t n = column[(int64_t)b * kDigits];
-      whole += n;
-      before += b < bis ? n : 0u;
+    for (int b = phase; b < blocks_per_segment; b += 4) {
+      const uint4 n = rows[b * (kDigits / 4) + quad];
+      whole.x += n.x;
+      whole.y += n.y;
+      whole.z += n.z;
+      whole.w += n.w;
+      if (b < bis) {
+        before.x += n.x;
+        before.y += n.y;
+        before.z += n.z;
+        before.w += n.w;
+      }
     }
+    reinterpret_cast<uint4*>(s_whole[phase])[quad] = whole;
+    reinterpret_cast<uint4*>(s_before[phase])[quad] = before;
   } else {
     block_offset[t] = offsets[((int64_t)seg * kDigits + t) * blocks_per_segment + bis];
   }
@@ -239,9 +257,12 @@ __global__ void __launch_bounds__(kSortThreads)
   }
   uint32_t block_total;
   digit_start[t] = block_exclusive_scan<uint32_t>(run, &block_total, warp_sums);
-  if (kCounting)
+  if constexpr (kCounting) {
+    const uint32_t whole = s_whole[0][t] + s_whole[1][t] + s_whole[2][t] + s_whole[3][t];
+    const uint32_t before = s_before[0][t] + s_before[1][t] + s_before[2][t] + s_before[3][t];
     block_offset[t] = (uint32_t)seg * blocks_per_segment * kTileItems + before +
                       block_exclusive_scan<uint32_t>(whole, &block_total, warp_sums);
+  }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
@@ -338,13 +359,14 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, ScanScratc
 namespace {
 
 // Items per thread of the counting passes, 0 where they do not pay: their blocks
-// each sum every block's counts of their view (up to 128 loads per thread) and
-// count each item with a global atomic, but a sort is 5 launches instead of 12 to
-// 20, and small tiles spread a small cloud over the SMs. The binning stage in us,
-// with and without: 60 / 78 (4k slots), 68 / 87 (20k), 90 / 126 (3 x 40k), 93 / 120
-// (60k), 124 / 131 (152k; 131 with 16 items), 173 / 184 (300k), 150 / 147 (400k).
+// each sum every block's counts of their view and count each item with a global
+// atomic, but a sort is 5 launches instead of 12 to 20, and small tiles spread a
+// small cloud over the SMs. The binning stage in us, with and without: 33 / 52 (4k
+// slots), 45 / 62 (20k), 64 / 91 (3 x 40k), 70 / 87 (60k), 109 / 129 (152k), 141 /
+// 154 (300k), 191 / 194 (600k); past the lines 244 / 237 (900k), and 597 / 475 for
+// 6M slots of 40 small views.
 int counting_items(int64_t segment_len, int64_t n) {
-  if (n > (int64_t)1 << 20 || segment_len > (int64_t)3 << 17) return 0;
+  if (n > (int64_t)1 << 20 || segment_len > (int64_t)5 << 17) return 0;
   return segment_len <= (int64_t)1 << 16 ? 4 : segment_len <= (int64_t)1 << 18 ? 8 : 16;
 }
 

@@ -24,8 +24,8 @@ def cloud_in_view(n, planes, seed):
     return p
 
 
-@pytest.mark.parametrize("n", [1, 31, 4095, 4096, 4097, 65536, 65537, 262144, 262145, 393216,
-                               393217])
+@pytest.mark.parametrize("n", [1, 31, 4095, 4096, 4097, 65536, 65537, 262144, 262145, 655360,
+                               655361])
 @pytest.mark.parametrize("planes", [0, 1, 37])
 def test_the_order_is_by_depth_then_index(n, planes):
     p = cloud_in_view(n, planes, n + planes)

@@ -1,12 +1,13 @@
 // param_grads.cu -- the backward parameter chain: per-(view, gaussian)
 // screen-space gradients back to each gaussian's parameters.
 //
-// rasterizeSplatsBackward, parameter pass (SplatRaster.cpp:435-575). One
-// thread per gaussian loops over the batch's views that render it (every
-// view for one cloud; its scene's views for a batch of several scenes),
-// keeping the parameter gradients in registers, and adds them into the
-// gradient array once. The
-// chain is gradient arithmetic, compiled with fused multiply-adds.
+// rasterizeSplatsBackward, parameter pass (SplatRaster.cpp:435-575). A batch of
+// one view runs a thread per gaussian; a larger one compacts the touched (view,
+// gaussian) slots of 128 gaussians, runs the chain a thread per slot and folds
+// each gaussian's slots in view order (every view for one cloud; its scene's
+// views for a batch of several scenes). Either way a gaussian's sums are added
+// into the gradient array once. The chain is gradient arithmetic, compiled with
+// fused multiply-adds.
 #include "common.cuh"
 #include "kernels.h"
 #include "project_common.cuh"
@@ -110,11 +111,10 @@ struct EntryLayout {
   static constexpr int kRows = PXS_C_SH_REST + S + 3;
 };
 
-// The parameter chain's shared memory (76 KB at SH degree 3).
+// The parameter chain's shared memory (53 KB at SH degree 3).
 template <int S>
 struct ParamSmem {
   static constexpr int kRest = 3 * S > 0 ? 3 * S : 1;
-  float coef[kRest][kParamThreads];  // sh_rest, channel-major
   float grad[kRest][kParamThreads];
   float acc[PXS_C_SH_REST][kParamThreads];
   float state[11][kParamThreads];  // position, unit quaternion, scales, raw norm
@@ -126,17 +126,17 @@ struct ParamSmem {
 
 // The chain of one touched (gaussian, view) slot (SplatRaster.cpp:455-575):
 // the gaussian's state (position, unit quaternion, its raw norm, scales), its
-// SH-rest coefficients `coef` (column of a [3S][kParamThreads] array) and the
-// slot's screen accumulators, projection and colour into the column `out`.
-template <int S>
+// SH-rest coefficients coef(j), and the slot's screen accumulators, projection
+// and colour into the column `out` (EntryLayout rows of kStride).
+template <int S, int kStride, typename Coef>
 __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4], const float sc[3],
-                                            float raw_norm, const float* coef,
+                                            float raw_norm, const Coef& coef,
                                             const ViewDesc& vd, const ScreenGrad& sg,
                                             const float4 co, const float4 col, float* out) {
   constexpr int kBasis0 = EntryLayout<S>::kBasis0;
   if constexpr (S > 0) {
 #pragma unroll
-    for (int b = 0; b < S; ++b) out[(kBasis0 + b) * kParamThreads] = 0.f;
+    for (int b = 0; b < S; ++b) out[(kBasis0 + b) * kStride] = 0.f;
   }
   float Rg[9], Mg[9], Sigma[9];
   rotation_from_unit(qn, Rg);
@@ -145,15 +145,15 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
   const uint32_t clamped = __float_as_uint(col.w);
   // opacity: alpha = sigmoid(logit) * G, dL/do = s0 / o
   const float opacity = co.w;
-  out[PXS_C_OPACITY * kParamThreads] = sg.s0 * (1.f - opacity);
+  out[PXS_C_OPACITY * kStride] = sg.s0 * (1.f - opacity);
   // colour: through the SH clamp into the coefficients and the direction
   float dcol[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     dcol[c] = sg.dcolor[c];
     if (clamped & (1u << c)) dcol[c] = 0.f;
-    out[(PXS_C_DC + c) * kParamThreads] = kShC0 * dcol[c];
-    out[(kBasis0 + S + c) * kParamThreads] = dcol[c];
+    out[(PXS_C_DC + c) * kStride] = kShC0 * dcol[c];
+    out[(kBasis0 + S + c) * kStride] = dcol[c];
   }
   float ddir[3] = {0.f, 0.f, 0.f};
   const int degree = vd.sh_degree;
@@ -175,9 +175,9 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
         if (b < usable) {
           float wb = 0.f;
 #pragma unroll
-          for (int c = 0; c < 3; ++c) wb += coef[(c * S + b) * kParamThreads] * dcol[c];
+          for (int c = 0; c < 3; ++c) wb += coef(c * S + b) * dcol[c];
           w[b] = wb;
-          out[(kBasis0 + b) * kParamThreads] = basis[b];
+          out[(kBasis0 + b) * kStride] = basis[b];
         }
       }
       sh_gradient_dot(usable, dir[0], dir[1], dir[2], w, ddir);
@@ -250,7 +250,7 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
     for (int i = 0; i < 3; ++i) dpos[i] += (ddir[i] - dir[i] * dd) / distance;
   }
 #pragma unroll
-  for (int i = 0; i < 3; ++i) out[(PXS_C_POSITION + i) * kParamThreads] = dpos[i];
+  for (int i = 0; i < 3; ++i) out[(PXS_C_POSITION + i) * kStride] = dpos[i];
   // Sigma = (R S)(R S)^T -> scale and rotation
   float sym2[9], dM[9];
 #pragma unroll
@@ -267,7 +267,7 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
   for (int a = 0; a < 3; ++a) {  // (R^T dM)(a, a) * s_a
     const float dS = dot3(Rg[0 * 3 + a], dM[0 * 3 + a], Rg[1 * 3 + a], dM[1 * 3 + a],
                           Rg[2 * 3 + a], dM[2 * 3 + a]);
-    out[(PXS_C_LOG_SCALE + a) * kParamThreads] = dS * sc[a];
+    out[(PXS_C_LOG_SCALE + a) * kStride] = dS * sc[a];
   }
   float dR[9];
 #pragma unroll
@@ -289,7 +289,7 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
   const float unit[4] = {qw, qx, qy, qz};
   const float ud = (unit[0] * dq[0] + unit[2] * dq[2]) + (unit[1] * dq[1] + unit[3] * dq[3]);
 #pragma unroll
-  for (int a = 0; a < 4; ++a) out[(PXS_C_ROTATION + a) * kParamThreads] = (dq[a] - unit[a] * ud) / raw_norm;
+  for (int a = 0; a < 4; ++a) out[(PXS_C_ROTATION + a) * kStride] = (dq[a] - unit[a] * ud) / raw_norm;
 }
 
 // Screen-space accumulators back to the gaussian's parameters
@@ -304,10 +304,16 @@ __device__ __forceinline__ void entry_chain(const float pos[3], const float qn[4
 // gaussian), compacts the touched (gaussian, view) entries by a block scan,
 // runs the chain on them with every lane busy, one entry per thread, and then
 // each thread folds its own gaussian's entries into its sums in view order
-// (deterministic: no atomics). The SH-rest coefficients and sums live in
-// shared memory.
+// (deterministic: no atomics).
+//
+// Bound by the latency of its reads at the warps it can hold. The SH-rest sums
+// live in shared memory; the coefficients are read from global memory by the
+// entry's thread (an owner's neighbours are mostly the next gaussians, so the
+// reads stay coalesced), because 23 KB less shared memory and 128 registers
+// hold 4 CTAs per SM instead of 3: 441 -> 374 us for 8 views of 1M gaussians,
+// 335 -> 281 for 40 views of 10 scenes, 44 -> 45 for 4 views of 100k.
 template <int S>
-__global__ void __launch_bounds__(kParamThreads, 3)
+__global__ void __launch_bounds__(kParamThreads, 4)
     k_param_grads(const float* __restrict__ params, int N, int64_t slot_stride,
                   const ViewDesc* __restrict__ views, int n_views, const uint32_t* depth_key,
                   const SlotGeom* __restrict__ geom, const float4* __restrict__ color,
@@ -317,7 +323,6 @@ __global__ void __launch_bounds__(kParamThreads, 3)
   constexpr int kBasis0 = EntryLayout<S>::kBasis0;
   extern __shared__ __align__(16) unsigned char param_smem[];
   ParamSmem<S>& sm = *reinterpret_cast<ParamSmem<S>*>(param_smem);
-  auto& s_coef = sm.coef;
   auto& s_grad = sm.grad;
   auto& s_acc = sm.acc;
   auto& s_state = sm.state;
@@ -371,14 +376,8 @@ __global__ void __launch_bounds__(kParamThreads, 3)
         // the first touched slot: the gaussian's state, its SH-rest
         // coefficients and cleared SH-rest sums
         if constexpr (S > 0) {
-          float coef[3 * S];
 #pragma unroll
-          for (int j = 0; j < 3 * S; ++j) coef[j] = params[(int64_t)(PXS_C_SH_REST + j) * N + g];
-#pragma unroll
-          for (int j = 0; j < 3 * S; ++j) {
-            s_coef[j][t] = coef[j];
-            s_grad[j][t] = 0.f;
-          }
+          for (int j = 0; j < 3 * S; ++j) s_grad[j][t] = 0.f;
         }
         GaussianState st;
         load_state(params, N, g, st);
@@ -429,8 +428,10 @@ __global__ void __launch_bounds__(kParamThreads, 3)
         const float qn[4] = {s_state[3][owner], s_state[4][owner], s_state[5][owner],
                              s_state[6][owner]};
         const float sc[3] = {s_state[7][owner], s_state[8][owner], s_state[9][owner]};
-        entry_chain<S>(pos, qn, sc, s_state[10][owner], &s_coef[0][owner], vd, sg, co, col,
-                       &s_res[0][t]);
+        entry_chain<S, T>(
+            pos, qn, sc, s_state[10][owner],
+            [=](int j) { return params[(int64_t)(PXS_C_SH_REST + j) * N + go]; }, vd, sg, co, col,
+            &s_res[0][t]);
       }
       __syncthreads();
       // each gaussian adds its entries of this chunk, in view order
@@ -477,6 +478,65 @@ __global__ void __launch_bounds__(kParamThreads, 3)
   }
 }
 
+// The same for a batch of one view, where a gaussian has one entry at most and
+// nothing is folded: a thread per gaussian with everything in registers, no
+// block-wide scan and no shared memory. What bounds it is the latency of three
+// dependent rounds of reads (slot, parameters, gradients). 56 -> 37 us for 152k
+// gaussians, 11 -> 9 for 20k, against the compacting kernel. It has no form for
+// more views: a thread whose neighbours have other touched views would idle,
+// and 45 SH-rest sums do not fit its registers.
+template <int S>
+__global__ void __launch_bounds__(kParamThreads)
+    k_param_grads_one(const float* __restrict__ params, int N, const ViewDesc* __restrict__ views,
+                      const uint32_t* __restrict__ depth_key, const SlotGeom* __restrict__ geom,
+                      const float4* __restrict__ color, const ScreenGrad* __restrict__ screen,
+                      float* __restrict__ grads, float* __restrict__ screen_gradient,
+                      int32_t* __restrict__ visible_count) {
+  constexpr int kBasis0 = EntryLayout<S>::kBasis0;
+  const int slot = blockIdx.x * kParamThreads + threadIdx.x;
+  const ViewDesc& vd = views[0];
+  if (slot >= vd.gauss_count || depth_key[slot] == kCulledKey) return;
+  const int g = vd.gauss_offset + slot;
+  const float4 tail = reinterpret_cast<const float4*>(screen + slot)[2];
+  visible_count[g] += 1;
+  screen_gradient[g] += tail.y;  // dmean_abs
+  if (tail.z == 0.f) return;     // no pixel past the alpha cap
+  const ScreenGrad sg = screen[slot];
+  const float4 co = geom[slot].conic_op, col = color[slot];
+  float coef[3 * S > 0 ? 3 * S : 1] = {};
+  if constexpr (S > 0) {
+#pragma unroll
+    for (int j = 0; j < 3 * S; ++j) coef[j] = params[(int64_t)(PXS_C_SH_REST + j) * N + g];
+  }
+  GaussianState st;
+  load_state(params, N, g, st);
+  float q[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) q[a] = params[(int64_t)(PXS_C_ROTATION + a) * N + g];
+  const float raw_norm = sqrtf((q[1] * q[1] + q[3] * q[3]) + (q[2] * q[2] + q[0] * q[0]));
+  float out[EntryLayout<S>::kRows];
+  entry_chain<S, 1>(st.pos, st.qn, st.s, raw_norm < 1e-12f ? 1e-12f : raw_norm,
+                    [&](int j) { return coef[j]; }, vd, sg, co, col, out);
+  // reads before writes, in groups
+  float old[PXS_C_SH_REST];
+#pragma unroll
+  for (int c = 0; c < PXS_C_SH_REST; ++c) old[c] = grads[(int64_t)c * N + g];
+#pragma unroll
+  for (int c = 0; c < PXS_C_SH_REST; ++c) grads[(int64_t)c * N + g] = old[c] + out[c];
+  if constexpr (S > 0) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      float rest[S];
+#pragma unroll
+      for (int b = 0; b < S; ++b) rest[b] = grads[(int64_t)(PXS_C_SH_REST + c * S + b) * N + g];
+#pragma unroll
+      for (int b = 0; b < S; ++b)
+        grads[(int64_t)(PXS_C_SH_REST + c * S + b) * N + g] =
+            rest[b] + __fmul_rn(out[kBasis0 + b], out[kBasis0 + S + c]);
+    }
+  }
+}
+
 void configure_param_grads_kernel() {
   cudaFuncSetAttribute(k_param_grads<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(ParamSmem<0>));
@@ -495,10 +555,15 @@ void launch_param_grads(const float* params, int N, int S, int64_t slot_stride,
                         cudaStream_t stream) {
   const int threads = kParamThreads;
   const int blocks = (N + threads - 1) / threads;
-  if (blocks == 0) return;
+  if (blocks == 0 || slot_stride == 0) return;
 #define LAUNCH(SS)                                                                      \
   count_launch();                                                                       \
-  k_param_grads<SS><<<blocks, threads, sizeof(ParamSmem<SS>), stream>>>(                \
+  if (n_views == 1)                                                                     \
+    k_param_grads_one<SS><<<(unsigned)((slot_stride + threads - 1) / threads), threads, 0, \
+                            stream>>>(params, N, views, depth_key, geom, color, screen, grads, \
+                                      screen_gradient, visible_count);                  \
+  else                                                                                  \
+    k_param_grads<SS><<<blocks, threads, sizeof(ParamSmem<SS>), stream>>>(                \
       params, N, slot_stride, views, n_views, depth_key, geom, color, screen, grads, \
       screen_gradient, visible_count)
   switch (S) {

@@ -379,15 +379,7 @@ int pxs_render(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* camer
     if (rgb == nullptr) throw Error(PXS_ERR_INVALID, "rgb is null");
     render_setup(ctx, cloud, camera, options, false);
     pxs::Frame& f = ctx->frame;
-    f.forward(ctx->stream);
-    const size_t pixels = static_cast<size_t>(f.batch.total_pixels);
-    if (pixels > 0) {
-      PXS_CUDA(cudaMemcpyAsync(rgb, f.rgb.get(), pixels * 3 * sizeof(float),
-                               cudaMemcpyDeviceToHost, ctx->stream));
-      if (transmittance)
-        PXS_CUDA(cudaMemcpyAsync(transmittance, f.transmittance.get(), pixels * sizeof(float),
-                                 cudaMemcpyDeviceToHost, ctx->stream));
-    }
+    f.forward_to_host(rgb, transmittance, ctx->stream);
     PXS_CUDA(cudaStreamSynchronize(ctx->stream));
   });
 }
@@ -441,19 +433,23 @@ int pxs_mean_ssim(pxs_context* ctx, const float* rendered, const float* target, 
   });
 }
 
-// Uploads host gradients, lets the kernels add into them, downloads them.
+// Uploads host gradients beside the kernels launched since begin_copies, lets the
+// parameter chain add into them, downloads them. (What a small call costs is its
+// pageable copies: 620 -> 555 us for 4k gaussians at 128x128, SH degree 3.)
 static void host_gradients_in(pxs_context* ctx, int P, int n, const pxs_gradients* g) {
   const size_t values = static_cast<size_t>(P) * static_cast<size_t>(n);
   float* d_grads = ctx->grads.reserve(values);
   float* d_screen = ctx->screen_gradient.reserve(static_cast<size_t>(n));
   int32_t* d_vis = ctx->visible_count.reserve(static_cast<size_t>(n));
   if (n == 0) return;
+  cudaStream_t copies = ctx->frame.copy_stream();
   PXS_CUDA(cudaMemcpyAsync(d_grads, g->params, values * sizeof(float), cudaMemcpyHostToDevice,
-                           ctx->stream));
+                           copies));
   PXS_CUDA(cudaMemcpyAsync(d_screen, g->screen_gradient, n * sizeof(float),
-                           cudaMemcpyHostToDevice, ctx->stream));
+                           cudaMemcpyHostToDevice, copies));
   PXS_CUDA(cudaMemcpyAsync(d_vis, g->visible_count, n * sizeof(int32_t), cudaMemcpyHostToDevice,
-                           ctx->stream));
+                           copies));
+  ctx->frame.join_copies(ctx->stream);
 }
 
 static void host_gradients_out(pxs_context* ctx, int P, int n, pxs_gradients* g) {
@@ -473,6 +469,14 @@ static void check_gradients(const pxs_gradients* g, int n) {
     throw Error(PXS_ERR_INVALID, "gradients are null");
 }
 
+// An image of the caller into `dst`, beside the kernels launched since begin_copies.
+static void host_image_in(pxs_context* ctx, float* dst, const float* src, size_t values) {
+  if (values == 0) return;
+  PXS_CUDA(cudaMemcpyAsync(dst, src, values * sizeof(float), cudaMemcpyHostToDevice,
+                           ctx->frame.copy_stream()));
+  ctx->frame.join_copies(ctx->stream);
+}
+
 int pxs_backward(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* camera,
                  const pxs_raster_options* options, const float* dL_drgb, pxs_gradients* grads) {
   return guarded(ctx, [&] {
@@ -481,16 +485,14 @@ int pxs_backward(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* cam
     const int P = PXS_PARAM_COUNT(cloud->rest_per_channel);
     render_setup(ctx, cloud, camera, options, false);
     pxs::Frame& f = ctx->frame;
-    f.forward(ctx->stream);
     const size_t values = static_cast<size_t>(f.batch.total_pixels) * 3;
     float* d_dL = ctx->dL.reserve(values);
-    if (values > 0) {
-      if (dL_drgb == nullptr) throw Error(PXS_ERR_INVALID, "dL_drgb is null");
-      PXS_CUDA(cudaMemcpyAsync(d_dL, dL_drgb, values * sizeof(float), cudaMemcpyHostToDevice,
-                               ctx->stream));
-    }
-    host_gradients_in(ctx, P, cloud->count, grads);
+    if (values > 0 && dL_drgb == nullptr) throw Error(PXS_ERR_INVALID, "dL_drgb is null");
+    f.begin_copies(ctx->stream);
+    f.forward(ctx->stream);
+    host_image_in(ctx, d_dL, dL_drgb, values);
     f.backward(d_dL, ctx->stream);
+    host_gradients_in(ctx, P, cloud->count, grads);
     f.param_grads(ctx->params.get(), ctx->grads.get(), ctx->screen_gradient.get(),
                   ctx->visible_count.get(), ctx->stream);
     host_gradients_out(ctx, P, cloud->count, grads);
@@ -509,16 +511,14 @@ int pxs_render_and_accumulate(pxs_context* ctx, const pxs_cloud* cloud, const px
     pxs::Frame& f = ctx->frame;
     const size_t values = static_cast<size_t>(f.batch.total_pixels) * 3;
     float* d_target = ctx->target.reserve(values);
-    if (values > 0) {
-      if (target == nullptr) throw Error(PXS_ERR_INVALID, "target is null");
-      PXS_CUDA(cudaMemcpyAsync(d_target, target, values * sizeof(float), cudaMemcpyHostToDevice,
-                               ctx->stream));
-    }
-    host_gradients_in(ctx, P, cloud->count, grads);
+    if (values > 0 && target == nullptr) throw Error(PXS_ERR_INVALID, "target is null");
+    f.begin_copies(ctx->stream);
     f.forward(ctx->stream);
     float* d_dL = ctx->dL.reserve(values);
+    host_image_in(ctx, d_target, target, values);
     f.loss(d_target, ssim_weight, 0, d_dL, ctx->stream);
     f.backward(d_dL, ctx->stream);
+    host_gradients_in(ctx, P, cloud->count, grads);
     f.param_grads(ctx->params.get(), ctx->grads.get(), ctx->screen_gradient.get(),
                   ctx->visible_count.get(), ctx->stream);
     host_gradients_out(ctx, P, cloud->count, grads);

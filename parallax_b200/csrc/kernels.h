@@ -138,12 +138,13 @@ void launch_tile_order(const int2* ranges, int total_tiles, int* order, int* wor
 // The forward pass; with two pixels per thread and `block_bits` given it also
 // writes, per tile-list entry, a byte whose bit b is set when some pixel of
 // the tile's 8x8 block b (b = 2 * row block + column block) took the entry.
-// Returns whether it wrote them.
+// Returns whether it wrote them. The two-pixel form in tile order may run the
+// tiles [first_tile, first_tile + total_tiles) only.
 bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                     int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                     cudaStream_t stream, unsigned long long* counts = nullptr,
                     uint8_t* block_bits = nullptr, const int* tile_order = nullptr,
-                    int* ticket = nullptr);
+                    int* ticket = nullptr, int first_tile = 0);
 // The adjoint. `block_bits`, when the forward wrote them, replace the
 // geometric warp masks in the two-pixel form: a warp walks only the entries
 // one of its pixels took.

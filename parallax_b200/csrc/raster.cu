@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(TileGeom<2>::kThreads, 8)
                  int n_views, float* __restrict__ rgb_out, float* __restrict__ T_out,
                  int32_t* __restrict__ last_out, unsigned long long* __restrict__ counts,
                  uint8_t* __restrict__ block_bits, int schedule, const int* __restrict__ order,
-                 int* __restrict__ ticket, int total_tiles) {
+                 int* __restrict__ ticket, int total_tiles, int first_tile) {
   constexpr int kThreads = TileGeom<2>::kThreads;
   __shared__ float2 s_xy[kFwdBatch];  // -mean
   __shared__ float4 s_co[kFwdBatch];  // conic, -opacity
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(TileGeom<2>::kThreads, 8)
   __shared__ uint8_t s_list[TileGeom<2>::kWarps][kFwdBatch];  // a warp's entries of the batch
   static_assert(kFwdBatch <= 256, "batch indices are bytes");
   for_each_tile(schedule, order, ticket, total_tiles, [&](int tile) {
-  const TileInfo<2> info = tile_info<2>(views, n_views, ranges, tile);
+  const TileInfo<2> info = tile_info<2>(views, n_views, ranges, first_tile + tile);
   const int warp = threadIdx.x >> 5;
   const ViewDesc& vd = views[info.view];
   const float min_alpha = vd.min_alpha, cutoff = vd.transmittance_cutoff;
@@ -395,7 +395,7 @@ template <bool kCount, bool kBits, int B>
 void forward_x2_launch(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                        int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                        cudaStream_t stream, unsigned long long* counts, uint8_t* bits,
-                       const int* order, int* ticket) {
+                       const int* order, int* ticket, int first_tile) {
   const RasterConfig& rc = raster_config();
   const int schedule = (kCount || order == nullptr) ? kTileOrder : rc.forward_schedule;
   int grid = total_tiles;
@@ -406,18 +406,18 @@ void forward_x2_launch(const int2* ranges, const uint32_t* pair_slots, const Slo
   }
   k_forward_x2<kCount, kBits, B><<<grid, TileGeom<2>::kThreads, 0, stream>>>(
       ranges, pair_slots, geom, color, views, n_views, rgb, T, last, counts, bits,
-      schedule, order, ticket, total_tiles);
+      schedule, order, ticket, total_tiles, first_tile);
 }
 
 template <bool kCount>
 void forward_x2_dispatch(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                          int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                          cudaStream_t stream, unsigned long long* counts, uint8_t* bits,
-                         const int* order, int* ticket) {
+                         const int* order, int* ticket, int first_tile) {
 #define PXS_FWD(BITS, B)                                                                    \
   forward_x2_launch<kCount, BITS, B>(ranges, pair_slots, geom, color, views, n_views, \
                                      total_tiles, rgb, T, last, stream, counts, bits, order,  \
-                                     ticket)
+                                     ticket, first_tile)
   const int b = raster_config().forward_batch;
   if (bits != nullptr) {
     if (b == 64) PXS_FWD(true, 64);
@@ -435,7 +435,7 @@ template <bool kCount>
 void forward_dispatch(int px, const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                       int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                       cudaStream_t stream, unsigned long long* counts, uint8_t* bits,
-                      const int* order, int* ticket) {
+                      const int* order, int* ticket, int first_tile) {
   switch (px) {
     case 1:
       forward_px<kCount, 1>(ranges, pair_slots, geom, color, views, n_views,
@@ -448,7 +448,7 @@ void forward_dispatch(int px, const int2* ranges, const uint32_t* pair_slots, co
     default:
       forward_x2_dispatch<kCount>(ranges, pair_slots, geom, color, views, n_views,
                                   total_tiles, rgb, T, last, stream, counts, bits, order,
-                                  ticket);
+                                  ticket, first_tile);
   }
 }
 
@@ -457,18 +457,19 @@ void forward_dispatch(int px, const int2* ranges, const uint32_t* pair_slots, co
 bool launch_forward(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,
                     int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                     cudaStream_t stream, unsigned long long* counts, uint8_t* block_bits,
-                    const int* tile_order, int* ticket) {
+                    const int* tile_order, int* ticket, int first_tile) {
   if (total_tiles <= 0) return false;
   count_launch();
   const int px = raster_config().forward_px;
   uint8_t* bits = (px == 1 || px == 4) ? nullptr : block_bits;
   if (counts != nullptr)
     forward_dispatch<true>(px, ranges, pair_slots, geom, color, views, n_views,
-                           total_tiles, rgb, T, last, stream, counts, bits, tile_order, ticket);
+                           total_tiles, rgb, T, last, stream, counts, bits, tile_order, ticket,
+                           first_tile);
   else
     forward_dispatch<false>(px, ranges, pair_slots, geom, color, views, n_views,
                             total_tiles, rgb, T, last, stream, nullptr, bits, tile_order,
-                            ticket);
+                            ticket, first_tile);
   return bits != nullptr;
 }
 

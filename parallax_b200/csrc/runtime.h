@@ -120,6 +120,8 @@ void ssim_kernel_weights(float out[11]);  // ssimKernel() with the host libm
 // Buffers and stages of one rasterisation batch: V views of an N-gaussian cloud.
 class Frame {
  public:
+  Frame() = default;
+  ~Frame();
   // Sizes the per-slot and per-pixel buffers and uploads the views.
   void prepare(const ViewBatch& batch, int N, int S, cudaStream_t stream);
   // Project every (view, gaussian) slot. The tile lists that bin() then builds
@@ -127,13 +129,23 @@ class Frame {
   // 3-sigma square, as the reference's do.
   void project(const float* params, cudaStream_t stream, bool debug_cov = false,
                bool whole_lists = false);
-  // Depth sort, pair emission, tile sort and ranges. With host_sync the pair
-  // count is read back and the pair buffers grown to fit; otherwise the
-  // preallocated capacity is used and an overflow raises the overflow flag.
+  // Depth sort and tile lists. With host_sync the pair count is read back and
+  // the pair buffers grown to fit; otherwise the preallocated capacity is used
+  // and an overflow raises the overflow flag.
   // Returns the pair count when synchronised, -1 otherwise.
   int64_t bin(bool host_sync, cudaStream_t stream);
   // counts (device, 2 values) receives evaluated and contributing pairs when given.
   void forward(cudaStream_t stream, unsigned long long* counts = nullptr);
+  // forward() of a batch of one view whose image goes to the host: bands of tile
+  // rows, each copied on the copy stream while the next ones are composited.
+  // `stream` waits for the copies. transmittance_out may be null.
+  void forward_to_host(float* rgb_out, float* transmittance_out, cudaStream_t stream);
+  // The copy stream of the calls on host memory. Copies issued on it follow what
+  // `stream` held at begin_copies(stream) and run beside what it is given after
+  // that, until it waits for them at join_copies(stream).
+  cudaStream_t copy_stream();
+  void begin_copies(cudaStream_t stream);
+  void join_copies(cudaStream_t stream);
   // Loss and dL/drgb against `target` (the batch's pixels, 3 floats each).
   void loss(const float* target, float ssim_weight, int mode, float* grad_out,
             cudaStream_t stream);
@@ -192,6 +204,9 @@ class Frame {
   uint32_t* sorted_slots = nullptr;
 
  private:
+  static constexpr int kMaxBands = 8;
+  cudaStream_t copy_stream_ = nullptr;
+  cudaEvent_t band_done_[kMaxBands] = {}, copied_ = nullptr;
   bool whole_lists_ = false;
   // Whether the tile lists are built directly (bin.cu).
   bool direct_lists() const;

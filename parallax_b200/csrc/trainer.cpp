@@ -1016,15 +1016,7 @@ int pxs_trainer_render(pxs_trainer* t, const pxs_camera* camera,
     t->frame.prepare(b, t->N, t->S, t->stream);
     t->frame.project(t->params.get(), t->stream);
     t->frame.bin(true, t->stream);
-    t->frame.forward(t->stream);
-    const size_t pixels = static_cast<size_t>(b.total_pixels);
-    if (pixels > 0) {
-      PXS_CUDA(cudaMemcpyAsync(rgb, t->frame.rgb.get(), pixels * 3 * sizeof(float),
-                               cudaMemcpyDeviceToHost, t->stream));
-      if (transmittance != nullptr)
-        PXS_CUDA(cudaMemcpyAsync(transmittance, t->frame.transmittance.get(),
-                                 pixels * sizeof(float), cudaMemcpyDeviceToHost, t->stream));
-    }
+    t->frame.forward_to_host(rgb, transmittance, t->stream);
     PXS_CUDA(cudaStreamSynchronize(t->stream));
   });
 }

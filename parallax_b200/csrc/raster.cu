@@ -152,15 +152,16 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
 // take an entry adds T * 0 * colour = 0.
 // kFwdBatch entries are staged per batch (RasterConfig::forward_batch: 64, 128
 // or 256; 128 by default -- a tile stops at saturation, so a smaller batch
-// stages fewer entries past it); `schedule` maps CTAs to tiles (for_each_tile).
-template <bool kCount, bool kBits, int kFwdBatch>
+// stages fewer entries past it); kPersist and `order` map CTAs to tiles
+// (for_each_tile).
+template <bool kCount, bool kBits, int kFwdBatch, bool kPersist>
 __global__ void __launch_bounds__(TileGeom<2>::kThreads, 8)
     k_forward_x2(const int2* __restrict__ ranges, const uint32_t* __restrict__ pair_slots,
                  const SlotGeom* __restrict__ geom,
                  const float4* __restrict__ color, const ViewDesc* __restrict__ views,
                  int n_views, float* __restrict__ rgb_out, float* __restrict__ T_out,
                  int32_t* __restrict__ last_out, unsigned long long* __restrict__ counts,
-                 uint8_t* __restrict__ block_bits, int schedule, const int* __restrict__ order,
+                 uint8_t* __restrict__ block_bits, const int* __restrict__ order,
                  int* __restrict__ ticket, int total_tiles, int first_tile) {
   constexpr int kThreads = TileGeom<2>::kThreads;
   __shared__ float2 s_xy[kFwdBatch];  // -mean
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(TileGeom<2>::kThreads, 8)
   __shared__ uint8_t s_took[TileGeom<2>::kWarps][kFwdBatch];  // warp w = 8x8 block w
   __shared__ uint8_t s_list[TileGeom<2>::kWarps][kFwdBatch];  // a warp's entries of the batch
   static_assert(kFwdBatch <= 256, "batch indices are bytes");
-  for_each_tile(schedule, order, ticket, total_tiles, [&](int tile) {
+  for_each_tile<kPersist>(order, ticket, total_tiles, [&](int tile) {
   const TileInfo<2> info = tile_info<2>(views, n_views, ranges, first_tile + tile);
   const int warp = threadIdx.x >> 5;
   const ViewDesc& vd = views[info.view];
@@ -396,17 +397,23 @@ void forward_x2_launch(const int2* ranges, const uint32_t* pair_slots, const Slo
                        int n_views, int total_tiles, float* rgb, float* T, int32_t* last,
                        cudaStream_t stream, unsigned long long* counts, uint8_t* bits,
                        const int* order, int* ticket, int first_tile) {
-  const RasterConfig& rc = raster_config();
-  const int schedule = (kCount || order == nullptr) ? kTileOrder : rc.forward_schedule;
-  int grid = total_tiles;
-  if (schedule == kPersistent) {
-    grid = std::min(total_tiles, resident_ctas(k_forward_x2<kCount, kBits, B>,
-                                               TileGeom<2>::kThreads));
-    cudaMemsetAsync(ticket, 0, sizeof(int), stream);
+  const int* tiles = kCount ? nullptr : order;
+  const int schedule = tiles == nullptr ? kTileOrder : raster_config().forward_schedule;
+  const int threads = TileGeom<2>::kThreads;
+  if constexpr (!kCount) {
+    if (schedule == kPersistent) {
+      const auto persistent = k_forward_x2<kCount, kBits, B, true>;
+      const int resident = resident_ctas(persistent, threads);
+      cudaMemsetAsync(ticket, 0, sizeof(int), stream);
+      persistent<<<std::min(total_tiles, resident), threads, 0, stream>>>(
+          ranges, pair_slots, geom, color, views, n_views, rgb, T, last, counts, bits, tiles,
+          ticket, total_tiles, first_tile);
+      return;
+    }
   }
-  k_forward_x2<kCount, kBits, B><<<grid, TileGeom<2>::kThreads, 0, stream>>>(
-      ranges, pair_slots, geom, color, views, n_views, rgb, T, last, counts, bits,
-      schedule, order, ticket, total_tiles, first_tile);
+  k_forward_x2<kCount, kBits, B, false><<<total_tiles, threads, 0, stream>>>(
+      ranges, pair_slots, geom, color, views, n_views, rgb, T, last, counts, bits, tiles, ticket,
+      total_tiles, first_tile);
 }
 
 template <bool kCount>

@@ -248,12 +248,12 @@ __device__ __forceinline__ uint32_t mask_from_block_bits(uint32_t bits) {
 // 2.81 ms over 40 views of ten small scenes, 0.131 -> 0.072 ms for one 320x240
 // view of 20k. Summing z, z d, z d^T d instead (seven lane sums, dx applied
 // once per column) ran in 4.39 ms but lost precision in elongated splats
-// (ScreenGrad); 9 or 10 CTAs per SM (56 or 48 registers, spills) in 4.80 and
-// 4.73 ms.
+// (ScreenGrad). 56 registers since each tile schedule has its own kernel: 4.50 ms
+// (for_each_tile); held to 48 (10 CTAs per SM) 4.57.
 // kB entries are staged per batch (RasterConfig::backward_batch: 64, 128 or
 // 256 with two pixels per thread; 128 with four, where fewer threads share a
-// batch); `schedule` maps CTAs to tiles (for_each_tile).
-template <int NP, int kB, bool kBits>
+// batch); kPersist and `order` map CTAs to tiles (for_each_tile).
+template <int NP, int kB, bool kBits, bool kPersist>
 __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
     k_backward_pairs(const int2* __restrict__ ranges, const uint32_t* __restrict__ pair_slots,
                      const SlotGeom* __restrict__ geom,
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
                      int n_views, const float* __restrict__ T_final,
                      const int32_t* __restrict__ last_in, const float* __restrict__ dL_drgb,
                      ScreenGrad* __restrict__ screen, const uint8_t* __restrict__ block_bits,
-                     int schedule, const int* __restrict__ order, int* __restrict__ ticket,
+                     const int* __restrict__ order, int* __restrict__ ticket,
                      int total_tiles) {
   constexpr int PX = 2 * NP;
   constexpr int kThreads = TileGeom<PX>::kThreads;
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
   __shared__ uint8_t s_list[kWarps][kB];  // a warp's entries of the batch
   __shared__ int s_hi;
   static_assert(kB <= 256, "batch indices are bytes");
-  for_each_tile(schedule, order, ticket, total_tiles, [&](int tile) {
+  for_each_tile<kPersist>(order, ticket, total_tiles, [&](int tile) {
   const TileInfo<PX> info = tile_info<PX>(views, n_views, ranges, tile);
   const ViewDesc& vd = views[info.view];
   const float min_alpha = vd.min_alpha;
@@ -471,15 +471,18 @@ void backward_pairs_launch(const int2* ranges, const uint32_t* pair_slots, const
                            cudaStream_t stream, const uint8_t* block_bits,
                            const int* tile_order, int* ticket) {
   const int schedule = tile_order == nullptr ? kTileOrder : raster_config().backward_schedule;
-  int grid = total_tiles;
+  const int threads = TileGeom<2 * NP>::kThreads;
   if (schedule == kPersistent) {
-    grid = std::min(total_tiles,
-                    resident_ctas(k_backward_pairs<NP, B, kBits>, TileGeom<2 * NP>::kThreads));
+    const auto persistent = k_backward_pairs<NP, B, kBits, true>;
     cudaMemsetAsync(ticket, 0, sizeof(int), stream);
+    persistent<<<std::min(total_tiles, resident_ctas(persistent, threads)), threads, 0, stream>>>(
+        ranges, pair_slots, geom, color, views, n_views, T_final, last, dL_drgb, screen,
+        block_bits, tile_order, ticket, total_tiles);
+  } else {
+    k_backward_pairs<NP, B, kBits, false><<<total_tiles, threads, 0, stream>>>(
+        ranges, pair_slots, geom, color, views, n_views, T_final, last, dL_drgb, screen,
+        block_bits, tile_order, ticket, total_tiles);
   }
-  k_backward_pairs<NP, B, kBits><<<grid, TileGeom<2 * NP>::kThreads, 0, stream>>>(
-      ranges, pair_slots, geom, color, views, n_views, T_final, last, dL_drgb, screen,
-      block_bits, schedule, tile_order, ticket, total_tiles);
 }
 
 void launch_backward(const int2* ranges, const uint32_t* pair_slots, const SlotGeom* geom, const float4* color, const ViewDesc* views,

@@ -77,29 +77,28 @@ inline int resident_ctas(Kernel kernel, int threads) {
 //                tile of that order from a device counter until none is left.
 enum TileSchedule { kTileOrder = 0, kHeavyFirst = 1, kPersistent = 2 };
 
-// Runs body(tile) for the tiles of this CTA under a schedule. `order` is the
-// heaviest-first tile order (schedules 1 and 2), `ticket` the counter of the
-// persistent schedule, zero at launch.
-template <typename Body>
-__device__ __forceinline__ void for_each_tile(int schedule, const int* __restrict__ order,
+// Runs body(tile) for the tiles of this CTA: the next ones of `order` (tile order
+// when null) by `ticket`, a counter that is zero at launch, or this CTA's one. A
+// template, because a kernel that held all three schedules behind a branch kept
+// more registers than the one it ran (64 for 56 in the adjoint): 4.60 -> 4.50 ms
+// in the adjoint and 2.26 -> 2.21 in the forward pass of 8 views of 1M gaussians,
+// 70 -> 66 us in the adjoint of 20k at 320x240.
+template <bool kPersist, typename Body>
+__device__ __forceinline__ void for_each_tile(const int* __restrict__ order,
                                               int* __restrict__ ticket, int total_tiles,
                                               Body&& body) {
-  if (schedule == kTileOrder) {
-    body((int)blockIdx.x);
-    return;
-  }
-  if (schedule == kHeavyFirst) {
-    body(order[blockIdx.x]);
-    return;
-  }
-  __shared__ int s_next;
-  for (;;) {
-    if (threadIdx.x == 0) s_next = atomicAdd(ticket, 1);
-    __syncthreads();
-    const int item = s_next;
-    __syncthreads();  // every thread has read it before thread 0 takes the next
-    if (item >= total_tiles) break;
-    body(order[item]);
+  if constexpr (!kPersist) {
+    body(order != nullptr ? order[blockIdx.x] : (int)blockIdx.x);
+  } else {
+    __shared__ int s_next;
+    for (;;) {
+      if (threadIdx.x == 0) s_next = atomicAdd(ticket, 1);
+      __syncthreads();
+      const int item = s_next;
+      __syncthreads();  // every thread has read it before thread 0 takes the next
+      if (item >= total_tiles) break;
+      body(order != nullptr ? order[item] : item);
+    }
   }
 }
 

@@ -33,7 +33,7 @@ struct ScanScratch {
 // `tight`: the tile rectangles cut to what a pixel can see of each splat.
 void launch_project(const float* params, int N, int S, int64_t slot_stride,
                     const ViewDesc* views, int n_views, const ProjectedSoA& out, bool tight,
-                    cudaStream_t stream);
+                    bool scenes, cudaStream_t stream);
 void configure_param_grads_kernel();  // once per device, outside graph capture
 void launch_param_grads(const float* params, int N, int S, int64_t slot_stride,
                         const ViewDesc* views, int n_views, const uint32_t* depth_key,

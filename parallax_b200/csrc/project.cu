@@ -21,7 +21,9 @@ constexpr int kProjectThreads = 256;
 // slot i holds gaussian gauss_offset + i of that view's range. Views of one
 // cloud share the gaussian, so its parameters are read once; a batch of
 // several scenes reads each scene's gaussian when the scene changes
-// (projectSplats, SplatRaster.cpp:201-258). The gaussian's S SH-rest
+// (projectSplats, SplatRaster.cpp:201-258). With a second grid dimension of one
+// block per view, the block of a run's first view takes the run -- neighbouring
+// views of one scene -- and the others return. The gaussian's S SH-rest
 // coefficients per channel are read together into this thread's column of
 // shared memory and serve every view.
 template <int S>
@@ -37,7 +39,14 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
   int g = -1;  // the gaussian whose state is loaded
   float dc0 = 0.f, dc1 = 0.f, dc2 = 0.f;
 
-  for (int v = 0; v < n_views; ++v) {
+  int v_begin = 0, v_end = n_views;
+  if (gridDim.y > 1) {
+    v_begin = blockIdx.y;
+    const int offset = views[v_begin].gauss_offset;
+    if (v_begin > 0 && views[v_begin - 1].gauss_offset == offset) return;
+    for (v_end = v_begin + 1; v_end < n_views && views[v_end].gauss_offset == offset;) ++v_end;
+  }
+  for (int v = v_begin; v < v_end; ++v) {
     const int64_t slot = v * slot_stride + i;
     const ViewDesc& vd = views[v];
     if (i >= vd.gauss_count) {
@@ -173,10 +182,14 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
 
 void launch_project(const float* params, int N, int S, int64_t slot_stride,
                     const ViewDesc* views, int n_views, const ProjectedSoA& out, bool tight,
-                    cudaStream_t stream) {
+                    bool scenes, cudaStream_t stream) {
   const int threads = kProjectThreads;
-  const int blocks = (int)((slot_stride + threads - 1) / threads);
-  if (blocks <= 0) return;
+  const unsigned slot_blocks = (unsigned)((slot_stride + threads - 1) / threads);
+  if (slot_blocks == 0 || n_views <= 0) return;
+  // A batch of scenes is sized by its largest one: a thread that walked every view
+  // would read one scene's gaussian after another (146 -> 105 us for 40 views of 10
+  // scenes, 460 -> 325 for 128 views of 32).
+  const dim3 blocks(slot_blocks, scenes && n_views <= 65535 ? (unsigned)n_views : 1u);
   count_launch();
   switch (S) {
     case 0:

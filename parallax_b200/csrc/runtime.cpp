@@ -217,7 +217,8 @@ void Frame::project(const float* params, cudaStream_t stream, bool want_debug,
   out.depth_key = depth_key.get();
   out.debug_cov = nullptr;
   if (want_debug) out.debug_cov = debug_cov.reserve(static_cast<size_t>(V) * slot_stride);
-  launch_project(params, N, S, slot_stride, d_views.get(), V, out, !whole_lists, stream);
+  launch_project(params, N, S, slot_stride, d_views.get(), V, out, !whole_lists,
+                 batch.own_ranges, stream);
   PXS_CUDA(cudaGetLastError());
 }
 

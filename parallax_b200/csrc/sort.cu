@@ -164,9 +164,25 @@ __global__ void __launch_bounds__(kSortThreads)
   }
 }
 
+// The lanes whose digit is this lane's, by a ballot per digit bit: __match_any_sync
+// takes a round per different digit, 47 against 18 us for a pass of 4M keys between
+// random digits and few. Binning 2.05 -> 1.98 ms at 8 views of 1M gaussians, 111 ->
+// 109 us at 152k. (The peers of all items first spare their chain, but 101
+// registers: 2.01 ms.)
+__device__ __forceinline__ unsigned digit_peers(uint32_t digit) {
+  unsigned peers = 0xffffffffu;
+#pragma unroll
+  for (int b = 0; b < kDigitBits; ++b) {
+    const bool bit = (digit >> b) & 1u;
+    const unsigned set = __ballot_sync(0xffffffffu, bit);
+    peers &= bit ? set : ~set;
+  }
+  return peers;
+}
+
 // Stable scatter of one block tile by one digit. Items are warp-striped (warp w
 // owns kItems * 32 consecutive ones, item k of a lane at k*32 + lane) and ranked
-// with __match_any_sync per digit, then offset by earlier warps. The tile is
+// among their digit's peers, then offset by earlier warps. The tile is
 // reordered by digit in shared memory and written out digit run by digit run,
 // so consecutive threads write consecutive addresses. vals_in null: the values
 // are the items' places.
@@ -238,7 +254,7 @@ __global__ void __launch_bounds__(kSortThreads)
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
     const uint32_t d = (key[k] >> shift) & (kDigits - 1);
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const unsigned peers = digit_peers(d);
     const uint32_t base = counts[warp * kDigits + d];
     __syncwarp();
     if (lane == __ffs(peers) - 1) counts[warp * kDigits + d] = base + __popc(peers);

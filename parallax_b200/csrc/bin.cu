@@ -434,18 +434,20 @@ __global__ void __launch_bounds__(kWarps * 32)
 // set bits' places, then takes a record per lane: its slot, and its columns cut
 // to the ones its splat reaches in that row (row_columns on shapes kept in shared
 // memory; without `tight` they stay the rectangle's). Bound by shared memory (the
-// shapes' reads meet random banks) at 3 CTAs per SM. Ranking in per-warp bitmaps
-// took 0.57 against 0.60 ms at 8 views of 1M gaussians, 1920x1440, but the binning
-// stage 446 against 423 us over 40 views of ten small scenes and 347 against 336
-// at 2 views of 700k, 1280x720.
+// shapes' reads meet random banks; in two arrays of halves eight lanes spread over
+// eight bank groups instead of four, the stage 1.98 -> 1.945 ms at 8 views of 1M) at
+// 3 CTAs per SM. Before that, ranking in per-warp bitmaps took 0.57 against 0.60 ms
+// at 8 views of 1M gaussians, 1920x1440, but the binning stage 446 against 423 us
+// over 40 views of ten small scenes and 347 against 336 at 2 views of 700k, 1280x720.
 constexpr int kMapRows = 512;
 struct RowExpandSmem {
-  RowShape shape[kSlotChunk];
+  float4 shape[2][kSlotChunk];         // the halves of the splats' RowShape
   uint32_t slot[kSlotChunk];
   uint16_t place[kWarps][kSlotChunk];  // a row's records: their splats' places
   uint32_t dst[kMapRows];              // each row's first record
 };
 static_assert(kSlotChunk == 32 * 32, "a word per lane");
+static_assert(sizeof(RowShape) == 32, "two 16-byte halves");
 
 __global__ void __launch_bounds__(kWarps * 32)
     k_slot_row_expand(const uint32_t* __restrict__ sorted_slots,
@@ -477,7 +479,10 @@ __global__ void __launch_bounds__(kWarps * 32)
       const Footprint f = splat_footprint(co, vd.min_alpha);
       shape = row_shape(f, co, geom[slot[k]].xy, xr[k]);
     }
-    sm.shape[place + k * 32] = shape;
+    float4 half[2];
+    memcpy(half, &shape, sizeof(shape));
+    sm.shape[0][place + k * 32] = half[0];
+    sm.shape[1][place + k * 32] = half[1];
   }
   const uint32_t cap = (uint32_t)capacity;  // at most 2^31 - 1
   for (int r0 = 0; r0 < tiles_y; r0 += kMapRows) {
@@ -512,7 +517,10 @@ __global__ void __launch_bounds__(kWarps * 32)
         if (dst + (uint32_t)i < cap) {
           const int p = sm.place[w][i];
           rec_slots[dst + i] = sm.slot[p];
-          rec_xr[dst + i] = row_columns(sm.shape[p], r0 + y);
+          const float4 half[2] = {sm.shape[0][p], sm.shape[1][p]};
+          RowShape shape;
+          memcpy(&shape, half, sizeof(shape));
+          rec_xr[dst + i] = row_columns(shape, r0 + y);
         }
       __syncwarp();  // the places are read before the next row's
     }

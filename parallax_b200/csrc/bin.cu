@@ -10,19 +10,17 @@
 //      within a row: each view's depth-sorted slots are cut into chunks of
 //      1024; a CTA per chunk counts, per tile row, the splats covering it; an
 //      exclusive scan of the counts in (row, chunk) order gives each chunk
-//      its base in each row, and the chunk writes its records there (the
-//      ranking of step 3 with rows for columns) -- a stable counting sort by
-//      row with no sort pass;
+//      its base in each row, and the chunk writes its records there (as in
+//      step 3 with rows for columns) -- a stable counting sort by row with no
+//      sort pass;
 //   2. each row is cut into chunks of 1024 records; one CTA per chunk counts,
 //      per column, the records covering it; a per-row pass turns those into
 //      each chunk's base within every tile of the row and the tiles' lengths;
 //      an exclusive scan over the tiles gives the tile ranges;
-//   3. one CTA per chunk walks its records again, 32 at a time per warp: each
-//      lane sets its bit in a per-column bitmap for every column its splat
-//      covers, and the pair's place among the chunk's pairs of that column is
-//      the column's running base plus the number of earlier lanes in the
-//      bitmap; the chunk's pairs are grouped by column in shared memory and
-//      copied out to the lists with consecutive stores.
+//   3. one CTA per chunk sets its records' bits in a 1024-bit map per column; a
+//      pair's place in its tile's list is the chunk's base plus the number of
+//      earlier bits of the column.
+// Images of few tiles skip the rows (Frame::direct_lists).
 // Over the splats' 3-sigma squares (Frame::project's whole_lists, for
 // pxs_tile_lists) the result -- ranges and slot lists -- is exactly the
 // reference's, with equal depths in gaussian order (the depth sort is stable over

@@ -178,6 +178,27 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   if (record_capacity > 0) ensure_chunks();
 }
 
+StepShape Frame::shape() const {
+  return {N,
+          S,
+          V,
+          slot_stride,
+          batch.own_ranges,
+          batch.total_pixels,
+          batch.total_tiles,
+          batch.total_rows,
+          batch.max_tiles,
+          batch.max_tiles_x,
+          batch.max_tiles_y,
+          batch.loss_rows,
+          batch.loss_blocks,
+          batch.l1_blocks,
+          pair_capacity,
+          record_capacity,
+          max_chunks,
+          direct_lists()};
+}
+
 void Frame::reserve_pairs(int64_t capacity) {
   if (capacity > INT32_MAX) throw Error(PXS_ERR_CAPACITY, "more than 2^31 tile pairs");
   if (capacity <= pair_capacity && tile_slots.get() != nullptr) return;

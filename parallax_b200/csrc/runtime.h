@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <cstring>
 #include <stdexcept>
@@ -117,6 +118,10 @@ ViewBatch make_batch(const pxs_camera* cameras, int n_views, const pxs_raster_op
 int bits_for(int64_t count);  // bits to represent values in [0, count)
 void ssim_kernel_weights(float out[11]);  // ssimKernel() with the host libm
 
+// Everything of a batch that sizes a launch or picks a kernel on the host
+// (Frame::shape).
+using StepShape = std::array<int64_t, 18>;
+
 // Buffers and stages of one rasterisation batch: V views of an N-gaussian cloud.
 class Frame {
  public:
@@ -124,6 +129,13 @@ class Frame {
   ~Frame();
   // Sizes the per-slot and per-pixel buffers and uploads the views.
   void prepare(const ViewBatch& batch, int N, int S, cudaStream_t stream);
+  // The prepared batch's shape. A captured graph of the stages holds the grids,
+  // shared memory sizes and branches of the shape it was captured for, and the
+  // view descriptors are read on the device: it stands for another batch only if
+  // the shapes are equal. (Equal pixels and tiles are not enough: 1402x1408 and
+  // 1408x1402 have both and different grids of the loss, 1280x720 and 720x1280
+  // different tile rows, scenes of one image size different slot strides.)
+  StepShape shape() const;
   // Project every (view, gaussian) slot. The tile lists that bin() then builds
   // hold the tiles a splat can reach, or with `whole_lists` every tile of its
   // 3-sigma square, as the reference's do.

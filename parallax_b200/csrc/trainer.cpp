@@ -29,9 +29,7 @@ namespace pxs {
 struct GraphState {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  int N = -1, V = -1;
-  int64_t pixels = -1, pair_capacity = -1, record_capacity = -1;
-  int tiles = -1;
+  StepShape shape{};  // Frame::shape() at capture
   int generation = -1;
   int raster_generation = -1;
   int64_t allocations = -1;
@@ -42,8 +40,6 @@ struct GraphState {
     if (graph != nullptr) cudaGraphDestroy(graph);
     exec = nullptr;
     graph = nullptr;
-    N = V = tiles = generation = raster_generation = -1;
-    pixels = pair_capacity = record_capacity = allocations = -1;
   }
 };
 
@@ -564,10 +560,8 @@ struct pxs_trainer {
     for (int attempt = 0; attempt < 3; ++attempt) {
       upload_scalars();
       if (use_graph) {
-        const bool stale = g.exec == nullptr || g.N != N || g.V != frame.V ||
-                           g.timing != timing || g.pixels != b.total_pixels ||
-                           g.tiles != b.total_tiles || g.pair_capacity != frame.pair_capacity ||
-                           g.record_capacity != frame.record_capacity ||
+        const pxs::StepShape shape = frame.shape();
+        const bool stale = g.exec == nullptr || g.shape != shape || g.timing != timing ||
                            g.generation != generation ||
                            g.raster_generation != pxs::raster_config().generation ||
                            g.allocations != pxs::g_device_allocations;
@@ -585,12 +579,7 @@ struct pxs_trainer {
           }
           PXS_CUDA(cudaStreamEndCapture(stream, &g.graph));
           PXS_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
-          g.N = N;
-          g.V = frame.V;
-          g.pixels = b.total_pixels;
-          g.tiles = b.total_tiles;
-          g.pair_capacity = frame.pair_capacity;
-          g.record_capacity = frame.record_capacity;
+          g.shape = shape;
           g.generation = generation;
           g.raster_generation = pxs::raster_config().generation;
           g.allocations = pxs::g_device_allocations;

@@ -168,11 +168,13 @@ __global__ void __launch_bounds__(kProjectThreads, 3)
         x1 = min(x1, last_tile(mean_x + f.ex));
         y0 = max(y0, first_tile(mean_y - f.ey));
         y1 = min(y1, last_tile(mean_y + f.ey));
-        if (x0 > x1 || y0 > y1) {  // no rows, no columns
-          x0 = y0 = 1;
-          x1 = y1 = 0;
-        }
       }
+    }
+    // No rows, no columns: nothing in reach, or a view without a pixel, whose last
+    // tile -1 would wrap to 65535.
+    if (x0 > x1 || y0 > y1) {
+      x0 = y0 = 1;
+      x1 = y1 = 0;
     }
     geom.rect = make_uint2((uint32_t)(x0 & 0xFFFF) | ((uint32_t)(x1 & 0xFFFF) << 16),
                            (uint32_t)(y0 & 0xFFFF) | ((uint32_t)(y1 & 0xFFFF) << 16));

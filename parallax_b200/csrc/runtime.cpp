@@ -269,6 +269,14 @@ int64_t Frame::bin(bool host_sync, cudaStream_t stream) {
   const uint32_t* const k = sort_keys.get();  // kCulledKey for a culled slot
   uint32_t* const v = sort_vals.get();
   sorted_slots = v;
+  if (batch.total_tiles == 0) {  // no view has a pixel: no lists
+    PXS_CUDA(cudaMemsetAsync(d_total_pairs.get(), 0, sizeof(int64_t), stream));
+    PXS_CUDA(cudaMemsetAsync(overflow.get(), 0, sizeof(int32_t), stream));
+    last_pair_count = last_record_count = 0;
+    sorted_pair_vals = tile_slots.get();
+    PXS_CUDA(cudaGetLastError());
+    return host_sync ? 0 : -1;
+  }
   if (direct_lists()) {
     launch_direct_counts(v, k, geom.get(), !whole_lists_, d_views.get(), V, slot_stride,
                          batch.max_tiles, batch.total_tiles, row_chunk_counts.get(),

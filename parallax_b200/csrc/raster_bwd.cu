@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(TileGeom<PX>::kThreads)
                 v.ww += zw * w;
                 v.u += zu;
                 v.w += zw;
-                v.ab += fabsf(z) * sqrt_approx_ftz(u * u + w * w);
+                v.ab += sqrt_approx_ftz(zu * zu + zw * zw);
               }
             }
           }
@@ -422,10 +422,11 @@ __global__ void __launch_bounds__(TileGeom<2 * NP>::kThreads)
         put(q, v.ww, zww.x + zww.y);
         put(q, v.u, zu.x + zu.y);
         put(q, v.w, zw.x + zw.y);
-        // |dL/dmean| per pixel, |z| |A d|, for the densification statistic (a
-        // sum compared against a threshold): the square-root approximation
-        const float2 sq = __ffma2_rn(u, u, __fmul2_rn(w, w));
-        put(q, v.ab, fabsf(z.x) * sqrt_approx_ftz(sq.x) + fabsf(z.y) * sqrt_approx_ftz(sq.y));
+        // |dL/dmean| per pixel, for the densification statistic (a sum compared
+        // against a threshold): the square-root approximation. Not |z| |A d|: in a
+        // splat of next to no width |A d|^2 overflows at pixels that have z = 0
+        const float2 sq = __ffma2_rn(zu, zu, __fmul2_rn(zw, zw));
+        put(q, v.ab, sqrt_approx_ftz(sq.x) + sqrt_approx_ftz(sq.y));
       }
     };
     // back to front, two entries at a time (one reduction serves both), then

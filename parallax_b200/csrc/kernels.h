@@ -155,17 +155,23 @@ void launch_backward(const int2* ranges, const uint32_t* pair_slots, const SlotG
                      int* ticket = nullptr);
 
 // loss.cu
-// CTAs of the loss over one image: `rows` output rows each (loss_rows), or with
-// rows = 0 the elementwise loss without SSIM.
-int64_t loss_blocks(int width, int height, int rows);
-// Output rows per CTA for these images together.
-int loss_rows(const int* widths, const int* heights, int n);
+void configure_loss_kernel();  // once per device, outside graph capture
+// How the loss runs: the elementwise form without SSIM; by tiles; or by CTAs that
+// march down `rows` output rows each.
+struct LossPlan {
+  enum Form { kL1, kTiles, kMarch };
+  Form form = kL1;
+  int rows = 0;
+};
+// The quickest form with SSIM for counts[k] images of each size k together.
+LossPlan loss_plan(const int* widths, const int* heights, const int* counts, int n);
+// CTAs of the loss over one image.
+int64_t loss_blocks(int width, int height, LossPlan plan);
 // One launch over every view's own CTAs, `blocks` in all, found by the views'
-// loss_tile_offset (rows > 0) or l1_block_offset (rows = 0). `sums`: 2 n_views + 1
-// doubles.
+// loss_tile_offset (l1_block_offset without SSIM). `sums`: 2 n_views + 1 doubles.
 void launch_loss(const float* rendered, const float* target, const ViewDesc* views, int n_views,
-                 int64_t blocks, int rows, const LossParams& lp, float* grad_out, double* sums,
-                 float* per_view, float* total, cudaStream_t stream);
+                 int64_t blocks, LossPlan plan, const LossParams& lp, float* grad_out,
+                 double* sums, float* per_view, float* total, cudaStream_t stream);
 
 // export.cu: the reference's file formats packed on the device
 void launch_pack_ply(const float* params, int n, const int* field_src, int fields, float* out,

@@ -18,6 +18,7 @@
 // the registers; only the strip's ten columns at either side and the march's
 // twenty extra rows are recomputed. Every blur sums in the reference's tap order;
 // the scalar totals are accumulated in double.
+// Batches too small for that go by 32x32 tiles (loss_plan).
 #include <algorithm>
 #include <cstdio>
 #include <exception>
@@ -288,6 +289,221 @@ __global__ void __launch_bounds__(kCols, 4)
   finish_loss<kCols>(l1_sum, ssim_sum, v, views, n_views, lp, sums, per_view, total);
 }
 
+// ---------------------------------------------------------------- small batches
+//
+// A march's rows follow one another, so a CTA takes (rows + 21) times a row's latency
+// however few CTAs there are: below about a megapixel in all, tiles finish first
+// (loss_plan). A CTA owns a 32x32 output tile and takes the channels one after
+// another: it stages a channel of both images over a 10-pixel halo, blurs the five
+// statistic planes onto a 5-pixel halo, forms the SSIM map and its partials there,
+// blurs those back onto the tile and writes the gradient. Each blur is register-
+// blocked: a thread loads a strip once and slides the 11 taps along it, in the
+// march's tap order. Bound by latency with one CTA on an SM, by instructions with two
+// (86 KB of shared memory each).
+constexpr int TW = 32, TH = 32;
+constexpr int IW = TW + 20, IH = TH + 20;  // input region
+constexpr int SW = TW + 10, SH = TH + 10;  // statistics region
+constexpr int kTileThreads = 320;  // every blur pass below is one round of items
+
+struct TileSmem {
+  float in_r[IH][IW];      // rendered, the current channel
+  float in_t[IH][IW];      // target
+  float hb[5][IH][SW];     // horizontal blur of the five products / of the three partials
+  float st[3][SH][SW];     // the three partial planes
+};
+
+__global__ void __launch_bounds__(kTileThreads, 2)
+    k_loss_tiles(const float* __restrict__ rendered, const float* __restrict__ target,
+                 const ViewDesc* __restrict__ views, int n_views, const LossParams lp,
+                 float* __restrict__ grad_out, double* __restrict__ sums,
+                 float* __restrict__ per_view, float* __restrict__ total) {
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  TileSmem& sm = *reinterpret_cast<TileSmem*>(tile_smem);
+  const int v = loss_view<false>(views, n_views, blockIdx.x);
+  const ViewDesc& vd = views[v];
+  const int W = vd.cam.width, H = vd.cam.height;
+  if (W <= 0 || H <= 0) {  // only where no view has a pixel
+    finish_loss<kTileThreads>(0.0, 0.0, v, views, n_views, lp, sums, per_view, total);
+    return;
+  }
+  const int local = blockIdx.x - vd.loss_tile_offset, across = (W + TW - 1) / TW;
+  const int ox = (local % across) * TW, oy = (local / across) * TH;
+  const int64_t pix0 = vd.pixel_offset;
+  const float* rimg = rendered + pix0 * 3;
+  const float* timg = target + vd.target_offset * 3;
+  const int tid = threadIdx.x;
+  const float w = lp.ssim_weight;
+  // 1 / values and 1 / (pixels * 3) of photometricLoss and meanSsim: equal
+  const float inv = 1.f / (float)((int64_t)W * H * 3);
+  const float c1 = 0.01f * 0.01f, c2 = 0.03f * 0.03f;
+  double l1_sum = 0.0, ssim_sum = 0.0;
+
+  for (int c = 0; c < 3; ++c) {
+    // stage channel c of both images over the input region, zero outside
+    // (the other channels' bytes of the same lines come back from L2)
+    for (int q = tid; q < IH * IW; q += kTileThreads) {
+      const int lx = q % IW, ly = q / IW;
+      const int X = ox - 10 + lx, Y = oy - 10 + ly;
+      float a = 0.f, b = 0.f;
+      if (X >= 0 && X < W && Y >= 0 && Y < H) {
+        const int64_t o = ((int64_t)Y * W + X) * 3 + c;
+        a = rimg[o];
+        b = timg[o];
+      }
+      sm.in_r[ly][lx] = a;
+      sm.in_t[ly][lx] = b;
+    }
+    __syncthreads();
+    // horizontal blur of the five products over every input row, onto the
+    // statistics columns; a thread slides the 11 taps over 7 outputs
+    constexpr int HS = 7;
+    for (int item = tid; item < IH * (SW / HS); item += kTileThreads) {
+      const int r = item / (SW / HS), col0 = (item % (SW / HS)) * HS;
+      float xs[HS + 10], ys[HS + 10], xx[HS + 10], yy[HS + 10], xy[HS + 10];
+#pragma unroll
+      for (int k = 0; k < HS + 10; ++k) {
+        xs[k] = sm.in_r[r][col0 + k];
+        ys[k] = sm.in_t[r][col0 + k];
+        xx[k] = xs[k] * xs[k];
+        yy[k] = ys[k] * ys[k];
+        xy[k] = xs[k] * ys[k];
+      }
+#pragma unroll
+      for (int o = 0; o < HS; ++o) {
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f, s4 = 0.f;
+#pragma unroll
+        for (int k = 0; k < 11; ++k) {
+          const float kk = lp.kernel[k];
+          s0 += kk * xs[o + k];
+          s1 += kk * ys[o + k];
+          s2 += kk * xx[o + k];
+          s3 += kk * yy[o + k];
+          s4 += kk * xy[o + k];
+        }
+        sm.hb[0][r][col0 + o] = s0;
+        sm.hb[1][r][col0 + o] = s1;
+        sm.hb[2][r][col0 + o] = s2;
+        sm.hb[3][r][col0 + o] = s3;
+        sm.hb[4][r][col0 + o] = s4;
+      }
+    }
+    __syncthreads();
+    // vertical blur -> statistics, then the SSIM map and its partials in
+    // place; a thread takes one column and 7 consecutive rows
+    constexpr int VS = 7;
+    constexpr int VSEG = (SH + VS - 1) / VS;
+    for (int item = tid; item < SW * VSEG; item += kTileThreads) {
+      const int col = item % SW, r0 = (item / SW) * VS;
+      float m[5][VS];
+#pragma unroll
+      for (int p = 0; p < 5; ++p) {
+        float hv[VS + 10];
+#pragma unroll
+        for (int k = 0; k < VS + 10; ++k) hv[k] = (r0 + k < IH) ? sm.hb[p][r0 + k][col] : 0.f;
+#pragma unroll
+        for (int o = 0; o < VS; ++o) {
+          float acc = 0.f;
+#pragma unroll
+          for (int k = 0; k < 11; ++k) acc += lp.kernel[k] * hv[o + k];
+          m[p][o] = acc;
+        }
+      }
+#pragma unroll
+      for (int o = 0; o < VS; ++o) {
+        const int r = r0 + o;
+        if (r >= SH) break;
+        const int X = ox - 5 + col, Y = oy - 5 + r;
+        float t_mu = 0.f, t_var = 0.f, t_cov = 0.f, mu_x = m[0][o], mu_y = m[1][o];
+        if (X >= 0 && X < W && Y >= 0 && Y < H) {
+          const float var_x = m[2][o] - mu_x * mu_x;
+          const float var_y = m[3][o] - mu_y * mu_y;
+          const float cov = m[4][o] - mu_x * mu_y;
+          const float a = 2.f * mu_x * mu_y + c1;
+          const float b = 2.f * cov + c2;
+          const float cc = mu_x * mu_x + mu_y * mu_y + c1;
+          const float d = var_x + var_y + c2;
+          // hardware reciprocal approximations (relative error ~1e-7, far
+          // inside the 1e-5 loss tolerance; cc >= C1 and d >= C2 - rounding)
+          const float rc = __fdividef(1.f, cc), rd = __fdividef(1.f, d);
+          const float r_ccd = rc * rd;  // 1 / (cc d)
+          const float ssim = (a * b) * r_ccd;
+          if (col >= 5 && col < 5 + TW && r >= 5 && r < 5 + TH) ssim_sum += (double)ssim;
+          t_mu = inv * (2.f * b * r_ccd) * (mu_y - mu_x * a * rc);
+          t_var = -inv * ssim * rd;
+          t_cov = inv * (2.f * a * r_ccd);
+        } else {
+          mu_x = 0.f;
+          mu_y = 0.f;
+        }
+        // dL/dx = blur(t_mu) + 2x blur(t_var) - 2 blur(t_var mu_x)
+        //        + y blur(t_cov) - blur(t_cov mu_y); the blur is linear, so
+        // the three terms without a pixel factor are blurred as one plane
+        sm.st[0][r][col] = t_mu - 2.f * t_var * mu_x - t_cov * mu_y;
+        sm.st[1][r][col] = t_var;
+        sm.st[2][r][col] = t_cov;
+      }
+    }
+    __syncthreads();
+    // horizontal blur of the partials onto the tile's columns, 16 per thread
+    constexpr int HS2 = 16;
+    for (int item = tid; item < 3 * SH * (TW / HS2); item += kTileThreads) {
+      const int p = item / (SH * (TW / HS2));
+      const int rem = item % (SH * (TW / HS2));
+      const int r = rem / (TW / HS2), col0 = (rem % (TW / HS2)) * HS2;
+      float tv[HS2 + 10];
+#pragma unroll
+      for (int k = 0; k < HS2 + 10; ++k) tv[k] = sm.st[p][r][col0 + k];
+#pragma unroll
+      for (int o = 0; o < HS2; ++o) {
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < 11; ++k) acc += lp.kernel[k] * tv[o + k];
+        sm.hb[p][r][col0 + o] = acc;
+      }
+    }
+    __syncthreads();
+    // vertical blur and the gradient, one column and 4 rows per thread
+    constexpr int VS2 = 4;
+    for (int item = tid; item < TW * (TH / VS2); item += kTileThreads) {
+      const int col = item % TW, r0 = (item / TW) * VS2;
+      float B[3][VS2];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        float hv[VS2 + 10];
+#pragma unroll
+        for (int k = 0; k < VS2 + 10; ++k) hv[k] = sm.hb[p][r0 + k][col];
+#pragma unroll
+        for (int o = 0; o < VS2; ++o) {
+          float acc = 0.f;
+#pragma unroll
+          for (int k = 0; k < 11; ++k) acc += lp.kernel[k] * hv[o + k];
+          B[p][o] = acc;
+        }
+      }
+#pragma unroll
+      for (int o = 0; o < VS2; ++o) {
+        const int r = r0 + o;
+        const int X = ox + col, Y = oy + r;
+        if (X >= W || Y >= H) continue;
+        const float x = sm.in_r[r + 10][col + 10];
+        const float y = sm.in_t[r + 10][col + 10];
+        float g = B[0][o];
+        g += 2.f * x * B[1][o];
+        g += y * B[2][o];
+        if (lp.mode == 0) {
+          const float diff = x - y;
+          l1_sum += (double)fabsf(diff);
+          const float sign = diff > 0.f ? 1.f : (diff < 0.f ? -1.f : 0.f);
+          g = (1.f - w) * sign * inv - w * g;
+        }
+        if (grad_out != nullptr) grad_out[(pix0 + (int64_t)Y * W + X) * 3 + c] = g;
+      }
+    }
+    __syncthreads();
+  }
+  finish_loss<kTileThreads>(l1_sum, ssim_sum, v, views, n_views, lp, sums, per_view, total);
+}
+
 // The loss without SSIM (w = 0): an elementwise pass, `rows` blocks of kL1Values
 // values per view's share of the grid. Bound by HBM (36 bytes per pixel).
 constexpr int kL1Threads = 256, kL1Values = 2048;
@@ -318,50 +534,91 @@ __global__ void __launch_bounds__(kL1Threads)
   finish_loss<kL1Threads>(l1_sum, 0.0, v, views, n_views, lp, sums, per_view, total);
 }
 
-int64_t loss_blocks(int width, int height, int rows) {
+int64_t loss_blocks(int width, int height, LossPlan plan) {
   if (width <= 0 || height <= 0) return 0;
-  if (rows <= 0) return ((int64_t)width * height * 3 + kL1Values - 1) / kL1Values;
-  return 3 * (int64_t)((width + kStrip - 1) / kStrip) * ((height + rows - 1) / rows);
+  switch (plan.form) {
+    case LossPlan::kL1:
+      return ((int64_t)width * height * 3 + kL1Values - 1) / kL1Values;
+    case LossPlan::kTiles:
+      return (int64_t)((width + TW - 1) / TW) * ((height + TH - 1) / TH);
+    default:
+      return 3 * (int64_t)((width + kStrip - 1) / kStrip) *
+             ((height + plan.rows - 1) / plan.rows);
+  }
 }
 
-// A march of R output rows takes R + 21 iterations. An iteration was measured at
-// 770, 950, 1300 and 1680 cycles with 1, 2, 3 and 4 CTAs on the SM (a row is a
-// chain of loads, blurs and a barrier that one CTA's four warps do not hide): short
-// marches spread small images over the SMs, long ones spare large images the
-// extra rows. R is the one with the least estimated time; at one view of 1280x720
-// 62 us, against 84 at 128 rows and 119 at 8, at 320x240 22 us against 36 at 48 (with
-// the order of summation before).
-int loss_rows(const int* widths, const int* heights, int n) {
-  constexpr int kSms = 148, kPerSm = 4;
-  constexpr double kCycles[kPerSm + 1] = {0.0, 770.0, 950.0, 1300.0, 1680.0};
-  int best = 8;
-  double best_cost = 0.0;
-  for (int rows = 8; rows <= 512; rows += std::max(4, rows / 32 * 4)) {
+namespace {
+
+// Estimated times in us, fitted to 134 batches of 1 to 64 images of 16 to 2000 pixels a
+// side. A march of R output rows takes R + 21 iterations of 960, 1120, 1460 or 1820
+// cycles with 1 to 4 CTAs on the SM (a row is a chain of loads, blurs and a barrier
+// that one CTA's four warps do not hide), 1680 in a wave that others follow: short
+// marches spread small batches over the SMs, long ones spare large ones the rows that
+// run in. Tiles take a round of a CTA on every SM after another.
+constexpr int kSms = 148;
+double march_us(int rows, int64_t blocks) {
+  constexpr int kPerSm = 4;
+  constexpr double kRow[kPerSm + 1] = {0.0, 960.0, 1120.0, 1460.0, 1820.0}, kFullRow = 1680.0;
+  constexpr double kCyclesPerUs = 1965.0;
+  const int64_t waves = blocks / (kSms * kPerSm), rest = blocks % (kSms * kPerSm);
+  return 7.0 + 4.0 * waves +
+         (rows + 21) / kCyclesPerUs * (waves * kFullRow + kRow[(rest + kSms - 1) / kSms]);
+}
+double tiles_us(int64_t blocks) {
+  return blocks <= kSms ? 24.5 : 11.7 + 10.9 * ((blocks + kSms - 1) / kSms);
+}
+
+}  // namespace
+
+// Tiles where the quickest march takes longer: one image of 541x541 in 33 us against 39,
+// two of 325x182 in 25 against 29, one of 110x2000 in 33 against 45 and eight of
+// 128x1000 in 91 against 109; the march one image of 320x240 in 23 against 25, one of
+// 1280x720 in 67 against 77.
+LossPlan loss_plan(const int* widths, const int* heights, const int* counts, int n) {
+  auto blocks_of = [&](LossPlan plan) {
     int64_t blocks = 0;
-    for (int v = 0; v < n; ++v) blocks += loss_blocks(widths[v], heights[v], rows);
-    const int64_t waves = blocks / (kSms * kPerSm), rest = blocks % (kSms * kPerSm);
-    const double cost =
-        (rows + 21) * (waves * kCycles[kPerSm] + kCycles[(rest + kSms - 1) / kSms]);
-    if (rows == 8 || cost < best_cost) {
-      best = rows;
-      best_cost = cost;
+    for (int k = 0; k < n; ++k)
+      blocks += (int64_t)counts[k] * loss_blocks(widths[k], heights[k], plan);
+    return blocks;
+  };
+  LossPlan best{LossPlan::kTiles, 0};
+  double best_us = tiles_us(blocks_of(best));
+  for (int rows = 8; rows <= 512; rows += std::max(4, rows / 32 * 4)) {
+    const LossPlan plan{LossPlan::kMarch, rows};
+    const double us = march_us(rows, blocks_of(plan));
+    if (us < best_us) {
+      best = plan;
+      best_us = us;
     }
   }
   return best;
 }
 
+void configure_loss_kernel() {
+  cudaFuncSetAttribute(k_loss_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)sizeof(TileSmem));
+}
+
 void launch_loss(const float* rendered, const float* target, const ViewDesc* views, int n_views,
-                 int64_t blocks, int rows, const LossParams& lp, float* grad_out, double* sums,
-                 float* per_view, float* total, cudaStream_t stream) {
+                 int64_t blocks, LossPlan plan, const LossParams& lp, float* grad_out,
+                 double* sums, float* per_view, float* total, cudaStream_t stream) {
   if (n_views <= 0) return;
   cudaMemsetAsync(sums, 0, sizeof(double) * (2 * n_views + 1), stream);
   count_launch();
-  if (rows > 0)
-    k_loss<<<(unsigned)std::max<int64_t>(blocks, 1), kCols, 0, stream>>>(rendered, target, views, n_views, lp, rows,
-                                                   grad_out, sums, per_view, total);
-  else
-    k_loss_l1<<<(unsigned)std::max<int64_t>(blocks, 1), kL1Threads, 0, stream>>>(rendered, target, views, n_views, lp,
-                                                           grad_out, sums, per_view, total);
+  const unsigned grid = (unsigned)std::max<int64_t>(blocks, 1);
+  switch (plan.form) {
+    case LossPlan::kL1:
+      k_loss_l1<<<grid, kL1Threads, 0, stream>>>(rendered, target, views, n_views, lp, grad_out,
+                                                 sums, per_view, total);
+      break;
+    case LossPlan::kTiles:
+      k_loss_tiles<<<grid, kTileThreads, sizeof(TileSmem), stream>>>(
+          rendered, target, views, n_views, lp, grad_out, sums, per_view, total);
+      break;
+    default:
+      k_loss<<<grid, kCols, 0, stream>>>(rendered, target, views, n_views, lp, plan.rows,
+                                         grad_out, sums, per_view, total);
+  }
 }
 
 }  // namespace pxs
@@ -417,12 +674,15 @@ struct StaticError {
 };
 
 // The scratch's device address on the current device; the first call on a
-// device looks it up.
+// device looks it up and raises the tiled kernel's shared-memory limit.
 StaticLossScratch* static_scratch(int device) {
   std::lock_guard<std::mutex> lock(g_scratch_mutex);
   if (g_scratch_addr[device] == nullptr) {
     void* ptr = nullptr;
     cudaError_t err = cudaGetSymbolAddress(&ptr, g_loss_scratch);
+    if (err != cudaSuccess) throw StaticError{PXS_ERR_CUDA, cudaGetErrorString(err)};
+    err = cudaFuncSetAttribute(k_loss_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(TileSmem));
     if (err != cudaSuccess) throw StaticError{PXS_ERR_CUDA, cudaGetErrorString(err)};
     g_scratch_addr[device] = static_cast<StaticLossScratch*>(ptr);
   }
@@ -476,12 +736,9 @@ extern "C" int pxs_photometric_loss_static(const float* rendered, const float* t
     StaticLossScratch* scratch = static_scratch(device);
     cudaGetLastError();  // an earlier, unrelated failure is not this call's
     count_launch();
-    int rows = 0;
-    if (ssim_weight > 0.f) {
-      const std::vector<int> ws(n_views, width), hs(n_views, height);
-      rows = loss_rows(ws.data(), hs.data(), n_views);
-    }
-    const int64_t blocks = loss_blocks(width, height, rows);
+    LossPlan plan;
+    if (ssim_weight > 0.f) plan = loss_plan(&width, &height, &n_views, 1);
+    const int64_t blocks = loss_blocks(width, height, plan);
     if (blocks * n_views > INT32_MAX) throw StaticError{PXS_ERR_INVALID, "images too large"};
     k_static_loss_views<<<(n_views + 63) / 64, 64, 0, s>>>(scratch, width, height, n_views,
                                                            (int)blocks);
@@ -490,7 +747,7 @@ extern "C" int pxs_photometric_loss_static(const float* rendered, const float* t
     lp.ssim_weight = ssim_weight;
     lp.mode = 0;
     // launch_loss clears scratch->sums on `s` before the kernel adds into them.
-    launch_loss(rendered, target, scratch->views, n_views, blocks * n_views, rows, lp, dL_drgb,
+    launch_loss(rendered, target, scratch->views, n_views, blocks * n_views, plan, lp, dL_drgb,
                 scratch->sums, per_view_loss, loss, s);
     err = cudaGetLastError();
     if (err != cudaSuccess) throw StaticError{PXS_ERR_CUDA, cudaGetErrorString(err)};

@@ -76,17 +76,24 @@ ViewBatch make_batch(const pxs_camera* cameras, int n_views, const pxs_raster_op
     b.max_tiles = std::max(b.max_tiles, d.tiles_x * d.tiles_y);
     pixel_offset += static_cast<int64_t>(d.cam.width) * d.cam.height;
   }
-  std::vector<int> widths, heights;
+  std::vector<int> widths, heights, counts;  // of the different sizes
   for (const ViewDesc& d : b.views) {
-    widths.push_back(d.cam.width);
-    heights.push_back(d.cam.height);
+    size_t k = 0;
+    while (k < counts.size() && (widths[k] != d.cam.width || heights[k] != d.cam.height)) ++k;
+    if (k == counts.size()) {
+      widths.push_back(d.cam.width);
+      heights.push_back(d.cam.height);
+      counts.push_back(0);
+    }
+    ++counts[k];
   }
-  b.loss_rows = loss_rows(widths.data(), heights.data(), n_views);
+  b.loss = loss_plan(widths.data(), heights.data(), counts.data(),
+                     static_cast<int>(counts.size()));
   for (ViewDesc& d : b.views) {
     d.loss_tile_offset = static_cast<int32_t>(b.loss_blocks);
     d.l1_block_offset = static_cast<int32_t>(b.l1_blocks);
-    b.loss_blocks += loss_blocks(d.cam.width, d.cam.height, b.loss_rows);
-    b.l1_blocks += loss_blocks(d.cam.width, d.cam.height, 0);
+    b.loss_blocks += loss_blocks(d.cam.width, d.cam.height, b.loss);
+    b.l1_blocks += loss_blocks(d.cam.width, d.cam.height, LossPlan{});
   }
   b.total_pixels = pixel_offset;
   b.total_tiles = tile_offset;
@@ -105,6 +112,7 @@ void Frame::ensure_scan_scratch(int64_t n) {
 
 void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   if (!configured_) {
+    configure_loss_kernel();
     configure_bin_kernels();
     configure_param_grads_kernel();
     PXS_CUDA(cudaGetLastError());
@@ -190,7 +198,8 @@ StepShape Frame::shape() const {
           batch.max_tiles,
           batch.max_tiles_x,
           batch.max_tiles_y,
-          batch.loss_rows,
+          batch.loss.form,
+          batch.loss.rows,
           batch.loss_blocks,
           batch.l1_blocks,
           pair_capacity,
@@ -466,7 +475,7 @@ void Frame::loss(const float* target, float ssim_weight, int mode, float* grad_o
   lp.mode = mode;
   const bool ssim = mode == 1 || ssim_weight > 0.f;
   launch_loss(rgb.get(), target, d_views.get(), V, ssim ? batch.loss_blocks : batch.l1_blocks,
-              ssim ? batch.loss_rows : 0, lp, grad_out, loss_sums.get(), loss_per_view.get(),
+              ssim ? batch.loss : LossPlan{}, lp, grad_out, loss_sums.get(), loss_per_view.get(),
               loss_total.get(), stream);
   PXS_CUDA(cudaGetLastError());
 }

@@ -95,7 +95,7 @@ struct ViewBatch {
   int total_rows = 0;       // tile rows over all views
   int max_tiles_x = 0, max_tiles_y = 0;
   int max_tiles = 0;        // of one view
-  int loss_rows = 0;        // output rows per CTA of the loss
+  LossPlan loss;            // of the loss with SSIM
   int64_t loss_blocks = 0, l1_blocks = 0;
   // the views carry their own gaussian ranges (several scenes); otherwise
   // Frame::prepare gives every view the whole cloud
@@ -120,7 +120,7 @@ void ssim_kernel_weights(float out[11]);  // ssimKernel() with the host libm
 
 // Everything of a batch that sizes a launch or picks a kernel on the host
 // (Frame::shape).
-using StepShape = std::array<int64_t, 18>;
+using StepShape = std::array<int64_t, 19>;
 
 // Buffers and stages of one rasterisation batch: V views of an N-gaussian cloud.
 class Frame {

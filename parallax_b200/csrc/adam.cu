@@ -38,6 +38,34 @@ __device__ __forceinline__ bool plain_scalars(const StepScalars& s) {
          isfinite(s.epsilon) && isfinite(s.correction1) && isfinite(s.correction2);
 }
 
+// Quaternion::norm / normalize over (x, y, z, w) storage (SplatTrainer.cpp:247-248).
+__device__ __forceinline__ void normalize(float (&q)[4]) {
+  const float sq = (q[1] * q[1] + q[3] * q[3]) + (q[2] * q[2] + q[0] * q[0]);
+  const float norm = sqrtf(sq);
+  if (norm > 1e-6f) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) q[a] = q[a] / norm;
+  } else {
+    q[0] = 1.f;
+    q[1] = q[2] = q[3] = 0.f;
+  }
+}
+
+// accumulateStatistics (SplatTrainer.cpp:258-263), then this step's stats clear.
+__device__ __forceinline__ void fold_statistics(int g, int zero_grads, float* screen_gradient,
+                                                int32_t* visible_count, float* acc_gradient,
+                                                int32_t* acc_views) {
+  if (screen_gradient == nullptr) return;
+  if (acc_gradient != nullptr) {
+    acc_gradient[g] += screen_gradient[g];
+    acc_views[g] += visible_count[g];
+  }
+  if (zero_grads) {
+    screen_gradient[g] = 0.f;
+    visible_count[g] = 0;
+  }
+}
+
 // The groups of V floats of the flat P x N arrays (k_adam). The rows' sections
 // end at floats 3N, 6N, 10N, 11N, 14N and P N: the first group that begins at
 // or past each end, and the group that straddles it (the largest Index: none).
@@ -52,7 +80,7 @@ struct AdamGroups {
 
 constexpr int kAdamThreads = 256, kAdamCtas = 6;
 
-// One kernel for every count and alignment. The parameters outside the rotation
+// The form for every count and alignment. The parameters outside the rotation
 // are one elementwise problem: the flat P x N arrays are cut into groups of V
 // consecutive floats (V = 4, 16-byte loads and stores, where the arrays start
 // on 16 bytes, whatever N is: groups run across rows), one group per thread,
@@ -66,7 +94,7 @@ constexpr int kAdamThreads = 256, kAdamCtas = 6;
 // reference's bits; 40 registers (6 CTAs per SM, a few bytes spilled around the
 // divisions' slow path) measured best. 333,333 gaussians SH3: 134.5 -> 102.3 us
 // (5.4 TB/s; rows of a count that is not a multiple of 4 took a gaussian per
-// thread before), 1M: 273.7 -> 266.2 us (6.2 TB/s).
+// thread before).
 template <int V>
 __global__ void __launch_bounds__(kAdamThreads, kAdamCtas)
     k_adam(float* __restrict__ params, float* __restrict__ grads, float* __restrict__ m,
@@ -101,29 +129,10 @@ __global__ void __launch_bounds__(kAdamThreads, kAdamCtas)
       v[i] = vv[a];
       if (zero_grads) grads[i] = 0.f;
     }
-    // Quaternion::norm / normalize over (x, y, z, w) storage (SplatTrainer.cpp:247-248)
-    const float sq = (q[1] * q[1] + q[3] * q[3]) + (q[2] * q[2] + q[0] * q[0]);
-    const float norm = sqrtf(sq);
-    if (norm > 1e-6f) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a) q[a] = q[a] / norm;
-    } else {
-      q[0] = 1.f;
-      q[1] = q[2] = q[3] = 0.f;
-    }
+    normalize(q);
 #pragma unroll
     for (int a = 0; a < 4; ++a) params[(PXS_C_ROTATION + a) * n + g] = q[a];
-    // accumulateStatistics (SplatTrainer.cpp:258-263), then this step's stats clear
-    if (screen_gradient != nullptr) {
-      if (acc_gradient != nullptr) {
-        acc_gradient[g] += screen_gradient[g];
-        acc_views[g] += visible_count[g];
-      }
-      if (zero_grads) {
-        screen_gradient[g] = 0.f;
-        visible_count[g] = 0;
-      }
-    }
+    fold_statistics(g, zero_grads, screen_gradient, visible_count, acc_gradient, acc_views);
     return;
   }
   // group k: floats [k V, k V + V); the groups wholly inside the rotation rows
@@ -183,6 +192,87 @@ __global__ void __launch_bounds__(kAdamThreads, kAdamCtas)
   }
 }
 
+// The same where N is a multiple of four and so every row starts on 16 bytes: no
+// group straddles two rows, and the rotation goes by groups too. A rotation block
+// takes 256 gaussians, a quarter of its threads per row; the new quaternions pass
+// through shared memory to a thread each, which normalises it, and back.
+//
+// 48 registers (5 CTAs per SM) without a spill: held to 40, its spills are on the way of
+// every thread (71 -> 82 us for 865,748 gaussians without SH). Times in us here / by
+// k_adam / a thread per gaussian group and row, with all four rotation rows in one
+// thread, cold and with the gradients cleared: 73 / 78 / 75 (865,748, no SH), 42 / 44 / 42
+// (400,000, no SH), 109 / 115 / 113 (865,748 SH1), 296 / 309 / 311 (1M SH3); it reaches
+// 6.2 TB/s at the last.
+constexpr int kRowsCtas = 5;
+
+__global__ void __launch_bounds__(kAdamThreads, kRowsCtas)
+    k_adam_rows(float* __restrict__ params, float* __restrict__ grads, float* __restrict__ m,
+                float* __restrict__ v, int N, int S, const StepScalars* __restrict__ scalars,
+                int zero_grads, float* __restrict__ screen_gradient,
+                int32_t* __restrict__ visible_count, float* __restrict__ acc_gradient,
+                int32_t* __restrict__ acc_views, const int32_t* __restrict__ skip,
+                const float* __restrict__ position_scale, int rot_blocks) {
+  __shared__ __align__(16) float s_q[4][kAdamThreads];
+  if (skip != nullptr && *skip != 0) return;
+  const StepScalars& s = *scalars;
+  const bool plain = plain_scalars(s);
+  const uint32_t n4 = (uint32_t)N / 4;
+  const bool rotation = (int)blockIdx.x < rot_blocks;
+  uint32_t k;  // the group
+  float lr;
+  bool live = true;
+  if (rotation) {
+    const uint32_t g4 = blockIdx.x * (kAdamThreads / 4) + threadIdx.x % (kAdamThreads / 4);
+    k = (PXS_C_ROTATION + threadIdx.x / (kAdamThreads / 4)) * n4 + g4;
+    lr = s.lr[2];
+    live = g4 < n4;
+  } else {
+    k = (blockIdx.x - rot_blocks) * kAdamThreads + threadIdx.x;
+    if (k >= PXS_C_ROTATION * n4) k += 4 * n4;
+    if (k >= (14 + 3 * S) * n4) return;
+    lr = k >= 14 * n4                ? s.lr[5]
+         : k >= 11 * n4              ? s.lr[4]
+         : k >= PXS_C_OPACITY * n4   ? s.lr[3]
+         : k >= PXS_C_LOG_SCALE * n4 ? s.lr[1]
+                                     : s.lr[0];
+  }
+  if (live) {
+    const float4 p4 = reinterpret_cast<const float4*>(params)[k];
+    const float4 g4 = reinterpret_cast<const float4*>(grads)[k];
+    const float4 m4 = reinterpret_cast<const float4*>(m)[k];
+    const float4 v4 = reinterpret_cast<const float4*>(v)[k];
+    float rate[4] = {lr, lr, lr, lr};
+    if (position_scale != nullptr && k < PXS_C_LOG_SCALE * n4) {
+      const float* at = position_scale + 4 * (k >= 2 * n4 ? k - 2 * n4 : k >= n4 ? k - n4 : k);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) rate[j] *= at[j];
+    }
+    float pp[4] = {p4.x, p4.y, p4.z, p4.w}, gg[4] = {g4.x, g4.y, g4.z, g4.w};
+    float mm[4] = {m4.x, m4.y, m4.z, m4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      pp[j] += adam_delta(mm[j], vv[j], gg[j], rate[j], s.beta1, s.beta2, s.epsilon,
+                          s.correction1, s.correction2, plain);
+    const float4 out = make_float4(pp[0], pp[1], pp[2], pp[3]);
+    if (rotation) reinterpret_cast<float4*>(s_q)[threadIdx.x] = out;
+    else reinterpret_cast<float4*>(params)[k] = out;
+    reinterpret_cast<float4*>(m)[k] = make_float4(mm[0], mm[1], mm[2], mm[3]);
+    reinterpret_cast<float4*>(v)[k] = make_float4(vv[0], vv[1], vv[2], vv[3]);
+    if (zero_grads) reinterpret_cast<float4*>(grads)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (!rotation) return;
+  __syncthreads();
+  const int t = threadIdx.x, g = blockIdx.x * kAdamThreads + t;
+  float q[4] = {s_q[0][t], s_q[1][t], s_q[2][t], s_q[3][t]};
+  normalize(q);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) s_q[a][t] = q[a];
+  __syncthreads();
+  if (live) reinterpret_cast<float4*>(params)[k] = reinterpret_cast<const float4*>(s_q)[t];
+  if (g < N)
+    fold_statistics(g, zero_grads, screen_gradient, visible_count, acc_gradient, acc_views);
+}
+
 namespace {
 
 template <int V>
@@ -208,13 +298,30 @@ void launch_adam_groups(float* params, float* grads, float* m, float* v, int N, 
       acc_gradient, acc_views, skip, position_scale, rot_blocks, groups);
 }
 
+void launch_adam_rows(float* params, float* grads, float* m, float* v, int N, int S,
+                      const StepScalars* scalars, int zero_grads, float* screen_gradient,
+                      int32_t* visible_count, float* acc_gradient, int32_t* acc_views,
+                      const int32_t* skip, cudaStream_t stream, const float* position_scale) {
+  const int rot_blocks = (N + kAdamThreads - 1) / kAdamThreads;
+  const int64_t groups = (10 + 3 * (int64_t)S) * (N / 4);
+  count_launch();
+  k_adam_rows<<<(unsigned)(rot_blocks + (groups + kAdamThreads - 1) / kAdamThreads),
+                kAdamThreads, 0, stream>>>(params, grads, m, v, N, S, scalars, zero_grads,
+                                           screen_gradient, visible_count, acc_gradient,
+                                           acc_views, skip, position_scale, rot_blocks);
+}
+
 template <typename... Args>
-void launch_adam_kernel(float* params, float* grads, float* m, float* v, Args... args) {
+void launch_adam_kernel(float* params, float* grads, float* m, float* v, int N, int S,
+                        Args... args) {
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-  if (aligned(params) && aligned(grads) && aligned(m) && aligned(v))
-    launch_adam_groups<4>(params, grads, m, v, args...);
+  const bool wide = aligned(params) && aligned(grads) && aligned(m) && aligned(v);
+  if (wide && N % 4 == 0)
+    launch_adam_rows(params, grads, m, v, N, S, args...);
+  else if (wide)
+    launch_adam_groups<4>(params, grads, m, v, N, S, args...);
   else
-    launch_adam_groups<1>(params, grads, m, v, args...);
+    launch_adam_groups<1>(params, grads, m, v, N, S, args...);
 }
 
 }  // namespace

@@ -414,11 +414,24 @@ void Frame::join_copies(cudaStream_t stream) {
   PXS_CUDA(cudaStreamWaitEvent(stream, copied_, 0));
 }
 
+// Whether the driver can copy to `p` directly (page-locked or device memory).
+static bool page_locked(const void* p) {
+  cudaPointerAttributes attributes;
+  if (cudaPointerGetAttributes(&attributes, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return attributes.type != cudaMemoryTypeUnregistered;
+}
+
 // A band is at least the tiles that the device composites at once (8 CTAs on
 // each of 148 SMs): with fewer the SMs would idle at every band's end. What the
 // copies take (31 MB of a 1600x1200 image at 52 GB/s: 590 us) hides the
 // compositing but for the first band's: a pinned 1600x1200 render of 300k
-// gaussians 1009 -> 910 us.
+// gaussians 1009 -> 910 us. A copy to pageable memory is staged by the host, which
+// fills and drains that pipeline for every band (20 to 50 us each): 20k gaussians at
+// 1600x1200, with the transmittance, took 1.79 ms in one band and 2.12 in eight, but
+// 12 Mpixels 8.01 and 7.75 ms, so there a band is also at least 1.25 Mpixels.
 void Frame::forward_to_host(float* rgb_out, float* transmittance_out, cudaStream_t stream) {
   constexpr int kBandTiles = 148 * 8;
   const RasterConfig& rc = raster_config();
@@ -426,6 +439,12 @@ void Frame::forward_to_host(float* rgb_out, float* transmittance_out, cudaStream
   int rows = tiles_y;
   if (V == 1 && rc.forward_px == 2 && rc.forward_schedule == 0 && tiles_x > 0)
     rows = std::max((kBandTiles + tiles_x - 1) / tiles_x, (tiles_y + kMaxBands - 1) / kMaxBands);
+  if (rows < tiles_y && !(page_locked(rgb_out) && (transmittance_out == nullptr ||
+                                                   page_locked(transmittance_out)))) {
+    constexpr int kBandPixels = 5 << 18;
+    const int bands = static_cast<int>(std::max<int64_t>(batch.total_pixels / kBandPixels, 1));
+    rows = std::max(rows, (tiles_y + bands - 1) / bands);
+  }
   const size_t pixels = static_cast<size_t>(batch.total_pixels);
   if (rows >= tiles_y || pixels == 0) {
     forward(stream);

@@ -31,6 +31,8 @@ struct pxs_context {
   DeviceArray<int32_t> export_fields;
   DeviceArray<uint8_t> ingest_in, ingest_bytes;
   DeviceArray<double> seed_nearest;
+  DeviceArray<pxs_projected_splat> projected;
+  DeviceArray<int32_t> projected_count;
 };
 
 namespace {
@@ -301,38 +303,19 @@ int pxs_project(pxs_context* ctx, const pxs_cloud* cloud, const pxs_camera* came
       throw Error(PXS_ERR_INVALID, "output is null");
     render_setup(ctx, cloud, camera, options, true);
     pxs::Frame& f = ctx->frame;
-    const size_t slots = static_cast<size_t>(f.slot_stride);
-    const auto order = download(f.sorted_slots, slots, ctx->stream);
-    const auto keys = download(f.depth_key.get(), slots, ctx->stream);
-    const auto geom = download(f.geom.get(), slots, ctx->stream);
-    const auto col = download(f.color.get(), slots, ctx->stream);
-    const auto cov = download(f.debug_cov.get(), slots, ctx->stream);
-    PXS_CUDA(cudaStreamSynchronize(ctx->stream));
+    // the most there can be; the slots past the cloud's are culled
+    pxs_projected_splat* d_out = ctx->projected.reserve(static_cast<size_t>(cloud->count));
+    int32_t* d_count = ctx->projected_count.reserve(1);
+    pxs::launch_projected_records(f.sorted_slots, f.sort_keys.get(), f.geom.get(), f.color.get(),
+                                  f.debug_cov.get(), f.slot_stride, d_out, d_count, ctx->stream);
+    PXS_CUDA(cudaGetLastError());
     int32_t n = 0;
-    for (size_t i = 0; i < slots; ++i) {
-      const uint32_t s = order[i];
-      if (keys[s] == pxs::kCulledKey) break;
-      pxs_projected_splat& p = out[n++];
-      p.index = static_cast<int32_t>(s);
-      p.mean[0] = geom[s].xy.x;
-      p.mean[1] = geom[s].xy.y;
-      p.cov2d[0] = cov[s].x;
-      p.cov2d[1] = cov[s].y;
-      p.cov2d[2] = cov[s].z;
-      p.radius = cov[s].w;
-      p.conic[0] = geom[s].conic_op.x;
-      p.conic[1] = geom[s].conic_op.y;
-      p.conic[2] = geom[s].conic_op.z;
-      p.opacity = geom[s].conic_op.w;
-      float depth;
-      std::memcpy(&depth, &keys[s], sizeof(float));
-      p.depth = depth;
-      p.color[0] = col[s].x;
-      p.color[1] = col[s].y;
-      p.color[2] = col[s].z;
-      uint32_t flags;
-      std::memcpy(&flags, &col[s].w, sizeof(uint32_t));
-      p.clamped = flags;
+    PXS_CUDA(cudaMemcpyAsync(&n, d_count, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+    PXS_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (n > 0) {
+      PXS_CUDA(cudaMemcpyAsync(out, d_out, sizeof(*out) * static_cast<size_t>(n),
+                               cudaMemcpyDeviceToHost, ctx->stream));
+      PXS_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     if (count) *count = n;
   });

@@ -34,6 +34,10 @@ struct ScanScratch {
 void launch_project(const float* params, int N, int S, int64_t slot_stride,
                     const ViewDesc* views, int n_views, const ProjectedSoA& out, bool tight,
                     bool scenes, cudaStream_t stream);
+// The visible slots of one view near to far, and their number (pxs_project).
+void launch_projected_records(const uint32_t* order, const uint32_t* keys, const SlotGeom* geom,
+                              const float4* color, const float4* cov, int64_t slots,
+                              pxs_projected_splat* out, int32_t* count, cudaStream_t stream);
 void configure_param_grads_kernel();  // once per device, outside graph capture
 void launch_param_grads(const float* params, int N, int S, int64_t slot_stride,
                         const ViewDesc* views, int n_views, const uint32_t* depth_key,

@@ -118,25 +118,6 @@ __device__ inline int warp_inclusive_scan(int v) {
   return v;
 }
 
-__device__ inline int warp_sum(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-__device__ inline float warp_sum(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Vector reduction to global memory (sm_90+): one L2 atomic for four floats.
-__device__ inline void red_add_v4(float* address, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(address), "f"(a), "f"(b),
-               "f"(c), "f"(d)
-               : "memory");
-}
-
 // Looks up which view of a batch a global tile belongs to (views are few).
 __device__ inline int view_of_tile(const ViewDesc* views, int n_views, int tile) {
   int v = 0;

@@ -427,9 +427,8 @@ int64_t finish_device(DensifyWork& w, const float* params, int N, int S, float m
   uint32_t* source = w.sort_b.reserve(n);
   uint32_t* buffers[4];
   for (int i = 0; i < 4; ++i) buffers[i] = w.sorted[i].reserve(static_cast<size_t>(padded));
-  const size_t hist_n = depth_sort_hist_entries(sorted, sorted);
-  uint32_t* hist = w.hist.reserve(hist_n);
-  uint32_t* hist_scanned = w.hist_scanned.reserve(hist_n);
+  uint32_t* hist = w.hist.reserve(depth_sort_hist_entries(sorted, sorted));
+  uint32_t* hist_scanned = w.hist_scanned.reserve(depth_sort_scanned_entries(sorted, sorted));
   count_launch();
   k_finish_keys<<<blocks, 256, 0, stream>>>(params, N, keep, keep_off, keys, source);
   PXS_CUDA(cudaMemsetAsync(keys + kept, 0xFF, sizeof(uint32_t) * (sorted - kept), stream));

@@ -54,9 +54,10 @@ void exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, ScanScratc
                         cudaStream_t stream);
 // Sorts n keys with their places as values, stably, each `segment_len` run
 // independently (both multiples of kSortTile), into keys_b and vals_b; the a
-// buffers are scratch, as are hist (depth_sort_hist_entries) and hist_scanned (as
-// large).
+// buffers are scratch, as are hist (depth_sort_hist_entries) and hist_scanned
+// (depth_sort_scanned_entries).
 size_t depth_sort_hist_entries(int64_t n, int64_t segment_len);
+size_t depth_sort_scanned_entries(int64_t n, int64_t segment_len);
 void depth_sort(const uint32_t* keys, int64_t n, int64_t segment_len, uint32_t* keys_a,
                 uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, uint32_t* hist,
                 uint32_t* hist_scanned, ScanScratch& scratch, cudaStream_t stream);

@@ -17,12 +17,6 @@ void check_cuda(cudaError_t err, const char* what) {
   }
 }
 
-int bits_for(int64_t count) {
-  int bits = 1;
-  while (bits < 40 && (int64_t(1) << bits) < count) ++bits;
-  return bits;
-}
-
 // ssimKernel (SplatRaster.cpp:587-600), with the same libm expf as the reference.
 void ssim_kernel_weights(float out[11]) {
   float total = 0.f;
@@ -151,7 +145,7 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
           ? static_cast<size_t>(std::max(batch.total_tiles, 1)) * direct_chunks_per_view(slot_stride)
           : static_cast<size_t>(std::max(batch.total_rows, 1)) * slot_chunks_per_view(slot_stride);
   row_chunk_counts.reserve(row_chunks);
-  row_chunk_offsets.reserve(row_chunks);
+  if (!direct_lists()) row_chunk_offsets.reserve(row_chunks);
   d_total_pairs.reserve(1);
   screen.reserve(slots);
   overflow.reserve(1);
@@ -172,11 +166,8 @@ void Frame::prepare(const ViewBatch& b, int n, int s, cudaStream_t stream) {
   loss_sums.reserve(static_cast<size_t>(2 * std::max(V, 1) + 1));
   loss_per_view.reserve(static_cast<size_t>(std::max(V, 1)));
   loss_total.reserve(1);
-  const size_t depth_hist = depth_sort_hist_entries(static_cast<int64_t>(slots), slot_stride);
-  if (hist.capacity() < depth_hist) {
-    hist.reserve(depth_hist);
-    hist_scanned.reserve(depth_hist);
-  }
+  hist.reserve(depth_sort_hist_entries(static_cast<int64_t>(slots), slot_stride));
+  hist_scanned.reserve(depth_sort_scanned_entries(static_cast<int64_t>(slots), slot_stride));
   ensure_scan_scratch(std::max<int64_t>(std::max<int64_t>(static_cast<int64_t>(slots),
                                                           static_cast<int64_t>(hist.capacity())),
                                         static_cast<int64_t>(

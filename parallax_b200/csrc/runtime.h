@@ -115,7 +115,6 @@ void downscaled_size(int width, int height, int target_width, int* out_width, in
 
 ViewBatch make_batch(const pxs_camera* cameras, int n_views, const pxs_raster_options& options,
                      int cloud_sh_degree);
-int bits_for(int64_t count);  // bits to represent values in [0, count)
 void ssim_kernel_weights(float out[11]);  // ssimKernel() with the host libm
 
 // Everything of a batch that sizes a launch or picks a kernel on the host

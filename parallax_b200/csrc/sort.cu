@@ -415,6 +415,11 @@ size_t depth_sort_hist_entries(int64_t n, int64_t segment_len) {
                    : (size_t)(n / kSortTile) * kDigits;
 }
 
+// The counting passes scan no counts.
+size_t depth_sort_scanned_entries(int64_t n, int64_t segment_len) {
+  return counting_items(segment_len, n) > 0 ? 0 : depth_sort_hist_entries(n, segment_len);
+}
+
 void depth_sort(const uint32_t* keys, int64_t n, int64_t segment_len, uint32_t* keys_a,
                 uint32_t* vals_a, uint32_t* keys_b, uint32_t* vals_b, uint32_t* hist,
                 uint32_t* hist_scanned, ScanScratch& scratch, cudaStream_t stream) {

@@ -43,6 +43,25 @@ struct GraphState {
   }
 };
 
+// The graphs of the last few shapes: batches of two or three shapes in turn (portrait
+// and landscape views, scenes of different size) replay one each. Capturing a step
+// costs 150 us.
+struct GraphPool {
+  static constexpr int kGraphs = 4;
+  GraphState graphs[kGraphs];
+  int oldest = 0;
+  GraphState& of(const StepShape& shape) {
+    for (GraphState& g : graphs)
+      if (g.exec != nullptr && g.shape == shape) return g;
+    GraphState& g = graphs[oldest];
+    oldest = (oldest + 1) % kGraphs;
+    return g;
+  }
+  void reset() {
+    for (GraphState& g : graphs) g.reset();
+  }
+};
+
 }  // namespace pxs
 
 using pxs::DeviceArray;
@@ -118,9 +137,9 @@ struct pxs_trainer {
   DeviceArray<pxs::StepScalars> scalars;
   DeviceArray<float> dL, loss_acc;
   std::string tune_log;       // the autotuner's timings, one line per candidate
-  pxs::GraphState graph;      // the batched step
-  pxs::GraphState graph_acc;  // its data-parallel accumulate half
-  pxs::GraphState graph_one;  // the one-view step (step())
+  pxs::GraphPool graph;      // the batched step
+  pxs::GraphPool graph_acc;  // its data-parallel accumulate half
+  pxs::GraphPool graph_one;  // the one-view step (step())
   bool pending_apply = false;
   int generation = 0;  // bumped whenever a state buffer is reallocated
   float* host_loss = nullptr;     // pinned
@@ -542,11 +561,11 @@ struct pxs_trainer {
                              cudaMemcpyDeviceToHost, stream));
   }
 
-  // Runs the batched body for `views`, replayed from `g` when use_graph, and
+  // Runs the batched body for `views`, replayed from a graph when use_graph, and
   // redoes it with larger pair buffers while the pairs overflow. The
   // optimiser, when included, skips a step whose pairs overflowed.
   void run_batch(const std::vector<int>& views, bool use_graph, bool with_adam,
-                 pxs::GraphState& g) {
+                 pxs::GraphPool& graphs) {
     const pxs::ViewBatch b = batch_for(views);
     frame.prepare(b, N, S, stream);  // also uploads the view descriptors
     dL.reserve(static_cast<size_t>(b.total_pixels) * 3 + 1);
@@ -561,6 +580,7 @@ struct pxs_trainer {
       upload_scalars();
       if (use_graph) {
         const pxs::StepShape shape = frame.shape();
+        pxs::GraphState& g = graphs.of(shape);
         const bool stale = g.exec == nullptr || g.shape != shape || g.timing != timing ||
                            g.generation != generation ||
                            g.raster_generation != pxs::raster_config().generation ||
@@ -606,7 +626,7 @@ struct pxs_trainer {
       const int64_t K = frame.bin(true, stream);
       frame.reserve_pairs(K + K / 2 + 65536);
       frame.reserve_records(frame.last_record_count + frame.last_record_count / 2 + 65536);
-      g.reset();
+      graphs.reset();
     }
     throw Error(PXS_ERR_CAPACITY, "tile pairs overflowed three times");
   }

@@ -111,3 +111,13 @@ def test_single_view_steps_of_scenes_of_other_counts():
         assert np.allclose(sorted(got), want, rtol=1e-5, atol=0)  # quaternions renormalised in between
     trainer.close()
     plain.close()
+
+
+@pytest.mark.parametrize("order", [[0, 1, 2, 3, 4, 5], [0, 1, 0, 2, 0, 3, 0, 4, 0, 5]])
+def test_more_shapes_than_graphs_are_kept(order):
+    # the graphs of the last four shapes are kept
+    params, rest = O.random_cloud(99, 4000, 1, log_scale_mean=-3.0)
+    cloud = px.GaussianCloud(params, 1, rest)
+    sizes = [(320, 240), (240, 320), (640, 120), (120, 640), (160, 480), (480, 160)]
+    pairs = [views(1, size, 40 + k)[0] for k, size in enumerate(sizes)]
+    compare(lambda: px.SplatTrainer(cloud, pairs, config()), [[k] for k in order])

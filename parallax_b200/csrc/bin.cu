@@ -359,9 +359,9 @@ __global__ void __launch_bounds__(kWarps * 32)
 // row, in depth order. Each view's depth-sorted slots are cut into chunks of
 // kSlotChunk; a chunk counts, per tile row of its view, the splats covering
 // it; an exclusive scan of those counts in (row, chunk) order gives every
-// chunk its base in every row; the chunk then writes its records there with
-// the same bitmap ranking and staging as the tile lists (rows for columns).
-// This is the stable counting sort of the records by row, with no sort pass.
+// chunk its base in every row; the chunk then sets its splats' bits in a
+// 1024-bit map per row and writes each row's records there in bit order. This
+// is the stable counting sort of the records by row, with no sort pass.
 constexpr int kSlotChunk = 1024;
 constexpr int kSlotPerLane = kSlotChunk / (kWarps * 32);  // slots per lane per chunk
 

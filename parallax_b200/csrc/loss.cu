@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kCols, 4)
       }
     }
     if (i == last_in) break;
-    // horizontal blur of x, y, x^2 + y^2 and x y
+    // horizontal blur of x, y, x^2, y^2 and x y
     float2 hxy = zero2, hsq = zero2;
     float hp = 0.f;
 #pragma unroll
@@ -504,8 +504,8 @@ __global__ void __launch_bounds__(kTileThreads, 2)
   finish_loss<kTileThreads>(l1_sum, ssim_sum, v, views, n_views, lp, sums, per_view, total);
 }
 
-// The loss without SSIM (w = 0): an elementwise pass, `rows` blocks of kL1Values
-// values per view's share of the grid. Bound by HBM (36 bytes per pixel).
+// The loss without SSIM (w = 0): an elementwise pass, a view's share of the grid
+// being one block per kL1Values of its values. Bound by HBM (36 bytes per pixel).
 constexpr int kL1Threads = 256, kL1Values = 2048;
 
 __global__ void __launch_bounds__(kL1Threads)
